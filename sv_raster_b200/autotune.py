@@ -15,9 +15,8 @@ gradients agree up to the order of floating-point additions):
 * ``sort`` -- segment-size buckets of the per-tile segment sort: the largest
   segment sorted by one small CTA and the chunk length of the chunked sort
   (``BatchedRasterizer.set_sort_buckets``).
-* ``reduce`` -- backward gradient reduction threshold: records touched by at
-  most this many lanes of a warp add their gradients with shared-memory
-  atomics instead of a warp reduce-scatter (``set_reduction``).
+* ``reduce`` -- ``set_reduction``'s argument, kept for choices saved with it
+  (the backward has one gradient reduction for any number of lanes).
 * ``bstage`` -- the backward's own staging depth (0: the forward's), tuned
   with the backward after the tile (``set_backward_staging``): the backward
   holds more per-record state in shared memory, so a shallower staging round
@@ -91,7 +90,7 @@ def _store_cache(path, data):
 
 # Bumped whenever the search space or the kernels behind it change, so that
 # choices cached by an older build are measured again rather than reused.
-CACHE_SCHEMA = 7
+CACHE_SCHEMA = 8
 
 
 def cache_key(raster, geos, sh0):

@@ -103,9 +103,9 @@ class BatchedRasterizer:
         self.binning = int(binning)
 
     def set_reduction(self, atomic_lanes=1):
-        """Backward: records with at most ``atomic_lanes`` contributing lanes
-        in a warp add their gradients with shared atomics instead of the warp
-        reduce-scatter (only the order of additions changes)."""
+        """Accepted (1 to 32) without effect: the backward sums every record's
+        gradients through rows in shared memory (see
+        svr_batch_plan_set_reduction)."""
         check(lib().svr_batch_plan_set_reduction(self.plan, int(atomic_lanes)), "batch_plan_set_reduction")
         self.atomic_lanes = int(atomic_lanes)
 

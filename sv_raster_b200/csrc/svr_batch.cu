@@ -64,47 +64,56 @@ project_sh_kernel(const __grid_constant__ ViewTable views, int P, const float* _
                   const float* __restrict__ lengths, const TS* __restrict__ sh0, const TS* __restrict__ shs, int M,
                   const int64_t* __restrict__ octpaths, int level_low_bits, int tight, uint32_t* __restrict__ ndup,
                   uint2* __restrict__ bboxes, uint32_t* __restrict__ quads, float* __restrict__ rgbs,
-                  uint32_t* __restrict__ err) {
+                  uint32_t* __restrict__ err, unsigned long long* __restrict__ pixels) {
   __shared__ float s_m[kMaxViews][24];           // w2c (12) and c2w (12) of every view
+  __shared__ unsigned long long s_pixels;
+  if (threadIdx.x == 0) s_pixels = 0ull;
   for (int t = threadIdx.x; t < views.n * 24; t += blockDim.x) {
     const int v = t / 24, k = t % 24;
     s_m[v][k] = k < 12 ? views.v[v].w2c[k] : views.v[v].c2w[k - 12];
   }
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P) return;
-  // voxels deeper than the plan's max level would break the compressed ranks
-  if (level_low_bits > 0 && ((uint64_t)octpaths[i] & ((1ull << level_low_bits) - 1ull)) != 0ull)
-    atomicOr(err, SVR_DEVERR_LEVEL);
-  const float cx = centers[3 * (size_t)i], cy = centers[3 * (size_t)i + 1], cz = centers[3 * (size_t)i + 2];
-  const float len = lengths[i];
-  // The rest coefficients are read per visible view through the cache
-  // (holding 45 of them in registers across the views cost the kernel half
-  // its occupancy).
-  const TS* sh = shs + (size_t)i * (M - 1) * 3;
-  float c0[3];
-  bool loaded = false;
-  for (int v = 0; v < views.n; ++v) {
-    const size_t o = (size_t)v * P + i;
-    const float* m = s_m[v];
-    Projection pr = project_voxel(views.v[v], m, m + 12, cx, cy, cz, len);
-    if (tight) tighten_bbox(views.v[v], pr);
-    ndup[o] = pr.n;
-    bboxes[o] = pr.bbox;
-    quads[o] = pr.quads;
-    if (pr.n == 0) continue;
-    if (!loaded) {
+  uint32_t px = 0u;  // bbox pixels over the views (each at most 2^20 here: a warp's sum fits 32 bits)
+  if (i < P) {
+    // voxels deeper than the plan's max level would break the compressed ranks
+    if (level_low_bits > 0 && ((uint64_t)octpaths[i] & ((1ull << level_low_bits) - 1ull)) != 0ull)
+      atomicOr(err, SVR_DEVERR_LEVEL);
+    const float cx = centers[3 * (size_t)i], cy = centers[3 * (size_t)i + 1], cz = centers[3 * (size_t)i + 2];
+    const float len = lengths[i];
+    // The rest coefficients are read per visible view through the cache
+    // (holding 45 of them in registers across the views cost the kernel half
+    // its occupancy).
+    const TS* sh = shs + (size_t)i * (M - 1) * 3;
+    float c0[3];
+    bool loaded = false;
+    for (int v = 0; v < views.n; ++v) {
+      const size_t o = (size_t)v * P + i;
+      const float* m = s_m[v];
+      Projection pr = project_voxel(views.v[v], m, m + 12, cx, cy, cz, len);
+      if (tight) tighten_bbox(views.v[v], pr);
+      ndup[o] = pr.n;
+      bboxes[o] = pr.bbox;
+      quads[o] = pr.quads;
+      if (pr.n == 0) continue;
+      if (!loaded) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) c0[c] = ldf(sh0, 3 * (size_t)i + c);
-      loaded = true;
+        for (int c = 0; c < 3; ++c) c0[c] = ldf(sh0, 3 * (size_t)i + c);
+        loaded = true;
+      }
+      // View-dependent colour of this visible voxel (sh_compute.cu:54-106).
+      float dx = cx - m[12 + 3], dy = cy - m[12 + 7], dz = cz - m[12 + 11];
+      const float rn = rnorm3df(dx, dy, dz);
+      dx = dx * rn; dy = dy * rn; dz = dz * rn;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) rgbs[3 * o + c] = sh_channel<DEG>(dx, dy, dz, c0[c], sh, c);
+      px += min((bb_xmax(pr.bbox) - bb_xmin(pr.bbox) + 1u) * (bb_ymax(pr.bbox) - bb_ymin(pr.bbox) + 1u), 1u << 20);
     }
-    // View-dependent colour of this visible voxel (sh_compute.cu:54-106).
-    float dx = cx - m[12 + 3], dy = cy - m[12 + 7], dz = cz - m[12 + 11];
-    const float rn = rnorm3df(dx, dy, dz);
-    dx = dx * rn; dy = dy * rn; dz = dz * rn;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) rgbs[3 * o + c] = sh_channel<DEG>(dx, dy, dz, c0[c], sh, c);
   }
+  px = __reduce_add_sync(0xffffffffu, px);
+  if ((threadIdx.x & 31) == 0 && px) atomicAdd(&s_pixels, (unsigned long long)px);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_pixels) atomicAdd(pixels + blockIdx.x % kCoverageSlots, s_pixels);
 }
 
 // Instance segment [start, start + count) of each sort group, clamped to the
@@ -384,7 +393,6 @@ struct svr_batch_plan {
   int tile_size;               // compositing tile size (8, 16 or 32), fixed at creation
   int stage;                   // records staged per round (svr_batch_plan_set_staging)
   int stage_bwd;               // the backward's, when set apart (svr_batch_plan_set_backward_staging)
-  int atomic_lanes;            // backward reduction threshold (svr_batch_plan_set_reduction)
   int exact;                   // compositing arithmetic (svr_batch_plan_set_arithmetic): 1 exact, 0 fast
   int pair;                    // two pixels per compositing thread (svr_batch_plan_set_pixels_per_thread)
   int pair_bwd;                // the backward's, when set apart (-1: as pair)
@@ -453,8 +461,13 @@ BatchPtrs ptrs(const svr_batch_plan* p, void* ws) {
 // Header words: [0] instance count, [1] error word, [2] forward work counter,
 // [3] backward work counter, [4] tile count read by the order sort, [5] pair
 // count read by the rank-position sort, [6] binned instance count (counting
-// sort by tile), [16..] group segments.
-constexpr int kHeaderWords = 16 + 2 * kMaxViews;
+// sort by tile), [16..] group segments, then the 64-bit pixel counts of
+// CoverageCount.
+constexpr int kCoverageWord = 16 + 2 * kMaxViews;
+constexpr int kHeaderWords = kCoverageWord + 2 * kCoverageSlots;
+unsigned long long* coverage_words(const BatchPtrs& q) {
+  return reinterpret_cast<unsigned long long*>(q.header + kCoverageWord);
+}
 
 // Longest-first work order of all tiles into `order` (see launch_tile_order).
 void build_tile_order(const svr_batch_plan* p, const BatchPtrs& q, const uint32_t* tile_last, uint32_t* order,
@@ -594,7 +607,6 @@ int svr_batch_plan_create(int n_views, const svr_camera* cams, int64_t P, int64_
   p->bwd_ctas_per_sm = 0;
   p->seg_small_n = 512;
   p->seg_chunk = 4096;
-  p->atomic_lanes = 1;
   p->exact = 0;
   p->pair = 0;
   p->pair_bwd = -1;
@@ -667,7 +679,6 @@ int svr_batch_plan_set_culling(svr_batch_plan* p, int culling) {
 
 int svr_batch_plan_set_reduction(svr_batch_plan* p, int atomic_lanes) {
   if (!p || atomic_lanes < 1 || atomic_lanes > 32) return SVR_ERR_SHAPE;
-  p->atomic_lanes = atomic_lanes;
   return SVR_OK;
 }
 
@@ -732,12 +743,12 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
   if (sh_bf16)                                                                                                \
     project_sh_kernel<D, __nv_bfloat16><<<pgrid, 128, 0, stream>>>(                                           \
         p->vt, P, vox_centers, vox_lengths, (const __nv_bfloat16*)sh0, (const __nv_bfloat16*)shs, M,         \
-        octree_paths, level_low, tight, q.ndup, q.bbox, q.quad, q.rgbs, q.header + 1);                        \
+        octree_paths, level_low, tight, q.ndup, q.bbox, q.quad, q.rgbs, q.header + 1, coverage_words(q));     \
   else                                                                                                        \
     project_sh_kernel<D, float><<<pgrid, 128, 0, stream>>>(p->vt, P, vox_centers, vox_lengths,               \
                                                            (const float*)sh0, (const float*)shs, M,          \
                                                            octree_paths, level_low, tight, q.ndup, q.bbox,   \
-                                                           q.quad, q.rgbs, q.header + 1);
+                                                           q.quad, q.rgbs, q.header + 1, coverage_words(q));
   const dim3 grid((P + 255) / 256, p->V);
   switch (sh_degree) {
     case 0: SVR_PROJ(0) break;
@@ -832,8 +843,7 @@ static int batch_backward(svr_batch_plan* p, void* ws, VoxelArrays va, const flo
   cudaMemsetAsync(q.drgbs, 0, (size_t)p->V * p->P * 16, stream);
   va.bboxes = q.bbox;
   va.rgbs = q.rgbs;
-  BwdTileIn in{out_T, q.ncontrib, dL_dcolor, nullptr, nullptr, dL_dT, nullptr, nullptr, 0.f, 0.f, 0.f,
-               p->atomic_lanes};
+  BwdTileIn in{out_T, q.ncontrib, dL_dcolor, nullptr, nullptr, dL_dT, nullptr, nullptr, 0.f, 0.f, 0.f};
   out.dL_drgbs = q.drgbs;
   out.err = q.header + 1;
   const bool ordered = (p->order_flags & 2) != 0;
@@ -841,7 +851,7 @@ static int batch_backward(svr_batch_plan* p, void* ws, VoxelArrays va, const flo
   launch_render_bwd_batch(p->vt, (int)p->total_tiles, q.ranges, q.tile_last, p->cap > 0 ? q.vb : nullptr, va,
                           (int)p->P, (size_t)p->P * 3, (size_t)p->P * 4, in, out, p->n_samp, p->tile_size,
                           p->stage_bwd, !p->exact, p->pair_bwd < 0 ? p->pair : p->pair_bwd,
-                          ordered ? q.order_bwd : nullptr, q.header + 3,
+                          CoverageCount{coverage_words(q), q.header}, ordered ? q.order_bwd : nullptr, q.header + 3,
                           p->bwd_ctas_per_sm, stream);
   return check_last();
 }

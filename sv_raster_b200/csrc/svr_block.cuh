@@ -35,6 +35,13 @@ __device__ __forceinline__ T block_exclusive_scan(T x, T* s_warp /*[NT/32]*/, T&
   return res;
 }
 
+// Place of the highest set bit (x != 0).
+__device__ __forceinline__ int bfind(uint32_t x) {
+  int r;
+  asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(x));
+  return r;
+}
+
 __device__ __forceinline__ uint32_t lanemask_lt() {
   uint32_t m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

@@ -35,13 +35,14 @@ struct Carver {
   size_t size() const { return align_up(off) + kAlign; }
 };
 
-// ---- geom buffer: header | n_dup | scan | bbox | quad | scan temp -------------
+// ---- geom buffer: header | n_dup | scan | bbox | quad | tight bbox | scan temp -------------
 struct GeomLayout {
   uint32_t* header;  // [0] instance count, [1] device error word
   uint32_t* ndup;
   uint32_t* scan;
   uint2* bbox;
   uint32_t* quad;
+  uint2* tight;      // pixel bbox that compositing tests (svr_preprocess.cu)
   void* scan_temp;
   size_t bytes;
 };
@@ -54,6 +55,7 @@ GeomLayout geom_layout(void* buf, int64_t P) {
   g.scan = c.take<uint32_t>(P);
   g.bbox = c.take<uint2>(P);
   g.quad = c.take<uint32_t>(P);
+  g.tight = c.take<uint2>(P);
   g.scan_temp = c.take<char>(scan_temp_bytes((size_t)P));
   g.bytes = c.size();
   return g;
@@ -241,7 +243,7 @@ int svr_rasterize_preprocess(const svr_camera* cam, int64_t P, const int64_t* oc
   vt.n = 1;
   vt.v[0] = make_view(*cam);
   cudaMemsetAsync(g.header, 0, 16 * sizeof(uint32_t), stream);
-  launch_preprocess(vt, (int)P, vox_centers, vox_lengths, out_n_duplicates, g.ndup, g.bbox, g.quad, stream);
+  launch_preprocess(vt, (int)P, vox_centers, vox_lengths, out_n_duplicates, g.ndup, g.bbox, g.quad, g.tight, stream);
   launch_scan_inclusive(g.ndup, g.scan, (size_t)P, g.scan_temp, g.header, 0xffffffffull, g.header + 1, stream);
   return check_launch(debug, stream);
 }
@@ -328,7 +330,7 @@ int svr_rasterize_render(const svr_camera* cam, int n_samp, int need_depth, int 
       (track_max_w && !max_w) || !geos || !rgbs || !vox_centers || !vox_lengths)
     return SVR_ERR_SHAPE;
   if (!aligned16(geos)) return SVR_ERR_ALIGN;
-  VoxelArrays va{c.g.bbox, vox_centers, vox_lengths, geos, nullptr, rgbs};
+  VoxelArrays va{c.g.tight, vox_centers, vox_lengths, geos, nullptr, rgbs};
   FwdTileOut out{c.im.tile_last, c.im.n_contrib, out_color, out_depth, out_normal, out_T, max_w};
   const uint32_t n_tiles = (uint32_t)(c.vt.v[0].grid_x * c.vt.v[0].grid_y);
   cudaMemsetAsync(c.im.tile_last, 0, n_tiles * sizeof(uint32_t), stream);  // combined by atomicMax
@@ -416,10 +418,10 @@ int svr_rasterize_backward(const svr_camera* cam, int n_samp, int64_t P, int64_t
   ImageLayout im = image_layout(const_cast<void*>(image_buffer), W, H);
   BinningLayout bl = binning_layout(const_cast<void*>(binning_buffer), (size_t)num_rendered, 0);
   const ViewParams vp = make_view(*cam);
-  VoxelArrays va{g.bbox, vox_centers, vox_lengths, geos, nullptr, rgbs};
+  VoxelArrays va{g.tight, vox_centers, vox_lengths, geos, nullptr, rgbs};
   BwdTileIn in{out_T, im.n_contrib, dL_dcolor, need_depth ? dL_ddepth : nullptr,
                need_normal ? dL_dnormal : nullptr, dL_dT, lambda_R_concen > 0 ? gt_color : nullptr,
-               need_dist ? out_depth : nullptr, lambda_R_concen, lambda_ascending, lambda_dist, 1};
+               need_dist ? out_depth : nullptr, lambda_R_concen, lambda_ascending, lambda_dist};
   BwdTileOut out{dL_dgeos, dL_drgbs, subdiv_p_bw, g.header + 1, aligned16(dL_dgeos) ? 1 : 0};
   // the forward's tile order (read only: the image buffer is the forward's saved state)
   launch_render_bwd(vp, im.ranges, im.tile_last, num_rendered > 0 ? bl.vals_b : nullptr, va, in, out, n_samp,
@@ -726,7 +728,7 @@ extern "C" int svr_rasterize_preprocess_noalloc(const svr_camera* cam, int64_t P
   vt.n = 1;
   vt.v[0] = make_view(*cam);
   cudaMemsetAsync(g.header, 0, 16 * sizeof(uint32_t), stream);
-  launch_preprocess(vt, (int)P, vox_centers, vox_lengths, out_n_duplicates, g.ndup, g.bbox, g.quad, stream);
+  launch_preprocess(vt, (int)P, vox_centers, vox_lengths, out_n_duplicates, g.ndup, g.bbox, g.quad, g.tight, stream);
   launch_scan_inclusive(g.ndup, g.scan, (size_t)P, partials, g.header, 0xffffffffull, g.header + 1, stream);
   return check_launch(debug, stream);
 }

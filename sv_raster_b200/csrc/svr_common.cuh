@@ -85,56 +85,65 @@ __device__ __forceinline__ uint32_t ray_quadrant(float dx, float dy, float dz) {
   return ((uint32_t)(dx < 0.f) << 2) | ((uint32_t)(dy < 0.f) << 1) | (uint32_t)(dz < 0.f);
 }
 
-// exp_linear_11 density activation and its derivative (auxiliary.h:278-286).
+// exp_linear_11 density activation (auxiliary.h:278-286).
 __device__ __forceinline__ float density_act(float x) {
   return (x > 1.1f) ? x : expf(0.909090909091f * x - 0.904689820196f);
 }
-__device__ __forceinline__ float density_act_grad(float x) {
-  return (x > 1.1f) ? 1.0f : 0.909090909091f * expf(0.909090909091f * x - 0.904689820196f);
+// Hardware exp2 and reciprocal (2 and 1 ulp; denormal results flush to zero)
+// and three-input minima and maxima that return NaN when an operand is NaN.
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
-
-// Both at once from a single expf: the same exponential the two functions
-// above evaluate separately, so the values are identical.
-__device__ __forceinline__ void density_act_and_grad(float x, float& act, float& grad) {
-  if (x > 1.1f) {
-    act = x;
-    grad = 1.0f;
-  } else {
-    const float e = expf(0.909090909091f * x - 0.904689820196f);
-    act = e;
-    grad = 0.909090909091f * e;
-  }
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float min3_nan(float a, float b, float c) {
+  float d;
+  asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
 }
 
 // Arithmetic of the compositing loops.  EXACT is the reference's own
 // operations (IEEE division, libdevice expf): contributor counts and images
-// come out bit-identical.  FAST uses the hardware exponential (ex2.approx of
-// x*log2(e), a few ulp) and an approximate division (reciprocal and multiply,
-// 2 ulp) for the per-(pixel, voxel) exponentials and the transmittance
-// recovery; results then differ from EXACT in the last bits, and a pixel may
-// stop one voxel earlier or later where T lands on the early-stop threshold.
+// come out bit-identical.  FAST uses the hardware exponential (exp2 with the
+// scale to base 2 folded into its argument, a few ulp) and an approximate
+// division (reciprocal and multiply, 2 ulp) for the per-(pixel, voxel)
+// exponentials and the transmittance recovery; results then differ from EXACT
+// in the last bits, and a pixel may stop one voxel earlier or later where T
+// lands on the early-stop threshold.
+constexpr float kLog2E = 1.4426950408889634f;
 template <bool FAST>
 __device__ __forceinline__ float exp_f(float x) {
-  return FAST ? __expf(x) : expf(x);
+  return FAST ? ex2_approx(x * kLog2E) : expf(x);
 }
 template <bool FAST>
 __device__ __forceinline__ float div_f(float a, float b) {
-  return FAST ? __fdividef(a, b) : a / b;
+  return FAST ? a * rcp_approx(b) : a / b;
+}
+// The exponential branch of the activation.
+template <bool FAST>
+__device__ __forceinline__ float act_exp_f(float x) {
+  return FAST ? ex2_approx(fmaf(0.909090909091f * kLog2E, x, -0.904689820196f * kLog2E))
+              : expf(0.909090909091f * x - 0.904689820196f);
 }
 template <bool FAST>
 __device__ __forceinline__ float density_act_f(float x) {
-  return (x > 1.1f) ? x : exp_f<FAST>(0.909090909091f * x - 0.904689820196f);
+  return (x > 1.1f) ? x : act_exp_f<FAST>(x);
 }
 template <bool FAST>
 __device__ __forceinline__ void density_act_and_grad_f(float x, float& act, float& grad) {
-  if (x > 1.1f) {
-    act = x;
-    grad = 1.0f;
-  } else {
-    const float e = exp_f<FAST>(0.909090909091f * x - 0.904689820196f);
-    act = e;
-    grad = 0.909090909091f * e;
-  }
+  const float e = act_exp_f<FAST>(x);
+  act = (x > 1.1f) ? x : e;
+  grad = (x > 1.1f) ? 1.0f : 0.909090909091f * e;
 }
 
 __device__ __forceinline__ float contract_depth(float x) {  // auxiliary.h:235-238
@@ -163,11 +172,17 @@ __device__ __forceinline__ void trilinear_weights(float qx, float qy, float qz, 
 struct PixelRay {
   float ox, oy, oz;      // origin (camera centre)
   float dx, dy, dz;      // unit direction (world)
-  float ix, iy, iz;      // 1 / direction
+  float ix, iy, iz;      // 1 / direction (+inf for a zero component, of either sign)
   float rd_norm_inv;     // 1 / |camera-space direction|
   uint32_t quad;         // octant of the direction
 };
 
+// Y_FIRST: which product of the direction's two-term dot products is rounded
+// before the other is fused onto it.  Written out so that every kernel agrees
+// with its counterpart (the compiler's choice differed between them): true is
+// the reference's order; the batched backward has always had the other one,
+// and its gradients (equally far from their exact values) keep it.
+template <bool Y_FIRST = true>
 __device__ __forceinline__ PixelRay make_pixel_ray(float pixx, float pixy, int W, int H,
                                                    float tanfovx, float tanfovy, float cx, float cy,
                                                    const float* c2w) {
@@ -180,9 +195,12 @@ __device__ __forceinline__ PixelRay make_pixel_ray(float pixx, float pixy, int W
   // compiler here picks the other operand (measured: images then differ
   // from the reference's in a few ulp at some pixels).
   const float rd_norm = sqrtf(__fmaf_rn(cdy, cdy, __fmul_rn(cdx, cdx)) + cdz * cdz);
-  const float rx = c2w[0] * cdx + c2w[1] * cdy + c2w[2] * cdz;
-  const float ry = c2w[4] * cdx + c2w[5] * cdy + c2w[6] * cdz;
-  const float rz = c2w[8] * cdx + c2w[9] * cdy + c2w[10] * cdz;
+  const auto dot2 = [&](float a, float b) {
+    return Y_FIRST ? __fmaf_rn(a, cdx, __fmul_rn(b, cdy)) : __fmaf_rn(b, cdy, __fmul_rn(a, cdx));
+  };
+  const float rx = dot2(c2w[0], c2w[1]) + c2w[2];
+  const float ry = dot2(c2w[4], c2w[5]) + c2w[6];
+  const float rz = dot2(c2w[8], c2w[9]) + c2w[10];
   r.rd_norm_inv = 1.f / rd_norm;
   r.ox = c2w[3];
   r.oy = c2w[7];
@@ -190,9 +208,11 @@ __device__ __forceinline__ PixelRay make_pixel_ray(float pixx, float pixy, int W
   r.dx = rx * r.rd_norm_inv;
   r.dy = ry * r.rd_norm_inv;
   r.dz = rz * r.rd_norm_inv;
-  r.ix = 1.f / r.dx;
-  r.iy = 1.f / r.dy;
-  r.iz = 1.f / r.dz;
+  // + 0 turns a -0 component into +0: the sign of the reciprocal then always
+  // agrees with the octant bit, which is what orders a slab's two planes.
+  r.ix = 1.f / (r.dx + 0.f);
+  r.iy = 1.f / (r.dy + 0.f);
+  r.iz = 1.f / (r.dz + 0.f);
   r.quad = ray_quadrant(r.dx, r.dy, r.dz);
   return r;
 }

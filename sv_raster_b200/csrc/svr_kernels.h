@@ -11,13 +11,20 @@
 namespace svr {
 
 struct VoxelArrays;
+// Pixels of the visible (view, voxel) pairs' bboxes, counted by the batched
+// projection over kCoverageSlots words, and the number of instances.
+constexpr int kCoverageSlots = 16;
+struct CoverageCount {
+  const unsigned long long* pixels;  // [kCoverageSlots]
+  const uint32_t* instances;
+};
 struct FwdTileOut;
 struct BwdTileIn;
 struct BwdTileOut;
 
 // svr_preprocess.cu
 void launch_preprocess(const ViewTable& views, int P, const float* centers, const float* lengths, int32_t* out_ndup,
-                       uint32_t* ndup, uint2* bboxes, uint32_t* quads, cudaStream_t stream);
+                       uint32_t* ndup, uint2* bboxes, uint32_t* quads, uint2* tight, cudaStream_t stream);
 
 // svr_binning.cu
 // Inclusive scan: CTAs of kScanThreads threads, kScanItems items each; the
@@ -88,7 +95,8 @@ void launch_render_bwd_batch(const ViewTable& views, int n_items, const uint2* r
                              const uint32_t* tile_last, const uint32_t* vals, const VoxelArrays& va, int P,
                              size_t rgb_view_stride, size_t drgb_view_stride, const BwdTileIn& in,
                              const BwdTileOut& out, int ns, int tile, int stage, bool fast, int pair,
-                             const uint32_t* order, uint32_t* counter, int ctas_per_sm, cudaStream_t stream);
+                             const CoverageCount& coverage, const uint32_t* order, uint32_t* counter, int ctas_per_sm,
+                             cudaStream_t stream);
 // svr_binning_deep.cu: binning of 21-level octrees (63-bit ranks).  The
 // sort pairs (keys_a, vals_a) / (keys_b, vals_b) and sort_temp are those of
 // the 16-level layout; vals_out / keys_lo are its sorted-value and sorted-key
@@ -111,6 +119,7 @@ void launch_binning_deep(const ViewParams& vp, int P, const int64_t* octpaths, c
                          uint32_t n, const DeepBinning& b, uint2* ranges, uint32_t* err, cudaStream_t stream);
 // Grid of a persistent launch: resident CTAs of `kernel` on this device
 // (capped at ctas_per_sm per SM when > 0), at most n_items.
+int sm_count();
 int persistent_grid(const void* kernel, int threads, size_t dyn_smem, int n_items, int ctas_per_sm);
 
 // svr_sh_adam.cu

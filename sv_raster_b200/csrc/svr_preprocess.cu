@@ -17,7 +17,8 @@ preprocess_kernel(const __grid_constant__ ViewTable views, int P,
                   int32_t* __restrict__ out_ndup,       // [V*P] or nullptr
                   uint32_t* __restrict__ ndup,          // [V*P]
                   uint2* __restrict__ bboxes,           // [V*P]
-                  uint32_t* __restrict__ quads)         // [V*P]
+                  uint32_t* __restrict__ quads,         // [V*P]
+                  uint2* __restrict__ tight)            // [V*P]: see below
 {
   const int view = blockIdx.y;
   const ViewParams& vp = views.v[view];
@@ -28,20 +29,30 @@ preprocess_kernel(const __grid_constant__ ViewTable views, int P,
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= P) return;
   const size_t o = (size_t)view * P + idx;
-  const Projection pr = project_voxel(vp, s_m, s_m + 12, centers[3 * (size_t)idx + 0], centers[3 * (size_t)idx + 1],
-                                      centers[3 * (size_t)idx + 2], lengths[idx]);
+  const float cx = centers[3 * (size_t)idx + 0], cy = centers[3 * (size_t)idx + 1], cz = centers[3 * (size_t)idx + 2];
+  Projection pr = project_voxel(vp, s_m, s_m + 12, cx, cy, cz, lengths[idx]);
   if (out_ndup) out_ndup[o] = (int32_t)pr.n;
   ndup[o] = pr.n;
   bboxes[o] = pr.bbox;
   quads[o] = pr.quads;
+  // The pixels whose rays can meet the voxel, for compositing alone (binning
+  // keeps the reference's rounded bbox, so the lists and their positions are the
+  // reference's): the records that a block then skips contribute nothing to it.
+  // On a 2M-voxel 1297x840 view this drops a third of the (record, pixel) pairs,
+  // and nearly all of them where the voxels are far smaller than a pixel.  The
+  // margin also covers the rounding of camera coordinates that are large against
+  // the voxel's depth.
+  const float reach = fabsf(cx) + fabsf(cy) + fabsf(cz) + fabsf(s_m[15]) + fabsf(s_m[19]) + fabsf(s_m[23]);
+  const float margin = kTightMargin + 1e-6f * fmaxf(vp.focal_x, vp.focal_y) * reach / fmaxf(pr.zmin, 1e-20f);
+  tight[o] = tighten_bbox(vp, pr, margin) ? pr.bbox : make_uint2(0xFFFFFFFFu, 0u);
 }
 
 void launch_preprocess(const ViewTable& views, int P, const float* centers, const float* lengths,
                        int32_t* out_ndup, uint32_t* ndup, uint2* bboxes, uint32_t* quads,
-                       cudaStream_t stream) {
+                       uint2* tight, cudaStream_t stream) {
   if (P <= 0 || views.n <= 0) return;
   dim3 grid((P + 255) / 256, views.n);
-  preprocess_kernel<<<grid, 256, 0, stream>>>(views, P, centers, lengths, out_ndup, ndup, bboxes, quads);
+  preprocess_kernel<<<grid, 256, 0, stream>>>(views, P, centers, lengths, out_ndup, ndup, bboxes, quads, tight);
 }
 
 }  // namespace svr

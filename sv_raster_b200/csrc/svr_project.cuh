@@ -18,11 +18,12 @@ struct Projection {
   uint32_t quads;  // camera-quadrant bitset (0 when culled)
   float bx0, by0, bx1, by1;  // the bbox before rounding (pixel coordinates, clamped to the image)
   bool front;                // all 8 corners in front of the near plane
+  float zmin;                // depth of the nearest corner (when front)
 };
 
 __device__ __forceinline__ Projection project_voxel(const ViewParams& vp, const float* w2c, const float* c2w,
                                                     float vcx, float vcy, float vcz, float len) {
-  Projection pr{0u, make_uint2(0u, 0u), 0u, 0.f, 0.f, 0.f, 0.f, false};
+  Projection pr{0u, make_uint2(0u, 0u), 0u, 0.f, 0.f, 0.f, 0.f, false, 0.f};
   const float vr = 0.5f * len;
   const float rox = c2w[3], roy = c2w[7], roz = c2w[11];
   const float near = vp.near_plane;
@@ -31,6 +32,7 @@ __device__ __forceinline__ Projection project_voxel(const ViewParams& vp, const 
   float umin = 1e9f, vmin = 1e9f, umax = -1e9f, vmax = -1e9f;
   uint32_t qbits = 0;
   int n_front = 0;
+  float zmin = 1e30f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float sx = (float)(((i & 4) >> 2) * 2 - 1);
@@ -47,6 +49,7 @@ __device__ __forceinline__ Projection project_voxel(const ViewParams& vp, const 
     umin = fminf(umin, u); vmin = fminf(vmin, v);
     umax = fmaxf(umax, u); vmax = fmaxf(vmax, v);
     qbits |= (1u << q);
+    zmin = fminf(zmin, camz);
     ++n_front;
   }
   const float cxh = vp.cx - 0.5f, cyh = vp.cy - 0.5f;
@@ -63,6 +66,7 @@ __device__ __forceinline__ Projection project_voxel(const ViewParams& vp, const 
   pr.quads = qbits;
   pr.bx0 = bx0; pr.by0 = by0; pr.bx1 = bx1; pr.by1 = by1;
   pr.front = n_front == 8;
+  pr.zmin = zmin;
   return pr;
 }
 
@@ -80,12 +84,12 @@ __device__ __forceinline__ Projection project_voxel(const ViewParams& vp, const 
 // centre remains (the voxel is culled for this view).
 constexpr float kTightMargin = 0.05f;
 
-__device__ __forceinline__ bool tighten_bbox(const ViewParams& vp, Projection& pr) {
+__device__ __forceinline__ bool tighten_bbox(const ViewParams& vp, Projection& pr, float margin = kTightMargin) {
   if (pr.n == 0 || !pr.front) return pr.n != 0;
-  const int x0 = max((int)bb_xmin(pr.bbox), (int)ceilf(pr.bx0 - kTightMargin));
-  const int y0 = max((int)bb_ymin(pr.bbox), (int)ceilf(pr.by0 - kTightMargin));
-  const int x1 = min((int)bb_xmax(pr.bbox), (int)floorf(pr.bx1 + kTightMargin));
-  const int y1 = min((int)bb_ymax(pr.bbox), (int)floorf(pr.by1 + kTightMargin));
+  const int x0 = max((int)bb_xmin(pr.bbox), (int)ceilf(pr.bx0 - margin));
+  const int y0 = max((int)bb_ymin(pr.bbox), (int)ceilf(pr.by0 - margin));
+  const int x1 = min((int)bb_xmax(pr.bbox), (int)floorf(pr.bx1 + margin));
+  const int y1 = min((int)bb_ymax(pr.bbox), (int)floorf(pr.by1 + margin));
   if (x0 > x1 || y0 > y1) {
     pr.n = 0;
     pr.quads = 0;

@@ -14,6 +14,7 @@
 
 #include <cuda_bf16.h>
 
+#include "svr_block.cuh"
 #include "svr_common.cuh"
 #include "svr_views.cuh"
 
@@ -37,24 +38,22 @@ struct TileCfg {
 // and composites each with four 8x8 CTAs that share the list.
 using PlainTile = TileCfg<8, 64>;
 constexpr int kPlainSub = 4;  // 8x8 CTAs per 16x16 list
+static_assert(PlainTile::SB <= PlainTile::NT, "ListReader stages one record per thread, and its ring holds two rounds");
 
 // Resident CTAs per SM the compositing kernels are register-bounded for at
-// 256 threads (64 registers each); other CTA sizes keep the same threads per
-// SM.  Chosen by measurement on the c4 step at 8x8 tiles: forward at 3 / 4 /
-// 5 / 6 gave 15.0 / 13.9 / 14.4 / 14.9 ms, backward at 3 / 4 / 5 gave
-// 31.2 / 29.0 / 41.6 ms.
+// 256 threads; other CTA sizes keep the same threads per SM.  The forward's was
+// chosen by measurement on the c4 step at 8x8 tiles: 3 / 4 / 5 / 6 gave 15.0 /
+// 13.9 / 14.4 / 14.9 ms.
 constexpr int kFwdMinBlocks = 4;
-constexpr int kBwdMinBlocks = 4;
+constexpr int kBwdMinBlocks = 3;
 template <class CFG>
 constexpr int fwd_min_blocks() { return CFG::NT >= 1024 ? 1 : kFwdMinBlocks * 256 / CFG::NT; }
+// The one-pixel backward: its CTAs of 64 threads run 13 (32 staged records) or
+// 11 (64) to an SM, at up to 78 or 90 registers (16 at 64 registers: the plain
+// backward 1.69 -> 2.08 ms on a 2M-voxel view).
 template <class CFG>
-constexpr int bwd_min_blocks() { return CFG::NT >= 1024 ? 1 : kBwdMinBlocks * 256 / CFG::NT; }
-// Backward with the distortion terms: its extra per-pixel state spills at the
-// 64-register budget (44-64 bytes), so those variants run one CTA fewer per
-// 256 threads (85 registers at 64-thread CTAs).
-template <class CFG, bool DIST>
-constexpr int bwd_min_blocks_for() {
-  return (DIST && CFG::NT < 1024) ? (kBwdMinBlocks - 1) * 256 / CFG::NT : bwd_min_blocks<CFG>();
+constexpr int bwd_min_blocks() {
+  return CFG::NT >= 1024 ? 1 : (CFG::NT == 64 ? (CFG::SB <= 32 ? 13 : 11) : kBwdMinBlocks * 256 / CFG::NT);
 }
 
 // Pixel of thread `tid` inside its tile: warp w owns micro-tile
@@ -82,26 +81,81 @@ struct VoxelArrays {
   const __nv_bfloat16* grid_bf16 = nullptr;
 };
 
-// One staged record.  Besides the raw attributes it holds the per-record
-// terms of the slab test and of the sample position, computed once here
-// instead of once per pixel: (c - o) -/+ l/2, c - l/2 and 1/l.  Each is the
-// same IEEE operation on the same operands as in the per-pixel form, so the
-// per-pixel results are unchanged bit for bit.
+// One staged record where lanes each read a record of their own (the forward,
+// and the backward with one pixel per thread).  Per-record terms of the slab
+// test and of the sample position are computed once here instead of once per
+// pixel, by the same IEEE operations on the same operands, so the per-pixel
+// results are unchanged bit for bit.  32 lanes on different records make a
+// 16-byte read cost 3.9 wavefronts on average, and wavefronts bound the forward
+// next to instruction issue (143 M of them and 638 M instructions in 196 M SM
+// cycles for 5.6 M instances): so a record is five 16-byte words to read, and
+// the two planes of each slab are formed per lane from (c - o, l/2).
 template <int SB>
-struct StageSmem {
-  uint4 box[SB];          // xmin, xmax - xmin, ymin, (ymax - ymin) | quadrant << 16
-  float4 slab_lo[SB];     // (c - o) - l/2 (xyz), 1/l (w)
-  float4 slab_hi[SB];     // (c - o) + l/2 (xyz), l (w)
-  float4 corner[SB];      // c - l/2 (xyz), voxel id as int bits (w)
-  float4 geo[SB][2];      // 8 corner densities
-  float4 rgb[SB];         // rgb (xyz)
+struct FwdStage {
+  uint4 box[SB];      // xmin, xmax - xmin, ymin, (ymax - ymin) | quadrant << 16
+  float4 rel[SB];     // c - o (xyz), l/2 (w)
+  float4 corner[SB];  // c - l/2 (xyz), 1/l (w)
+  float4 geo[SB][2];  // 8 corner densities, or their polynomial (fast arithmetic)
+  float4 rgb[SB];     // rgb (xyz), voxel id as int bits (w)
 };
+
+// One staged record of the two-pixel backward, whose lanes all read the same
+// record (one wavefront per word): the slab's planes are staged in the order
+// in which rays of the record's octant cross them.
+template <int SB>
+struct BwdStage {
+  uint4 box[SB];      // as in FwdStage
+  float4 near[SB];    // (c - o) -/+ l/2 (xyz), the plane crossed first; 1/l (w)
+  float4 far[SB];     // (c - o) +/- l/2 (xyz), the other
+  float4 corner[SB];  // c - l/2 (xyz), voxel id as int bits (w)
+  float4 geo[SB][2];  // 8 corner densities, or their polynomial (fast arithmetic)
+  float4 rgb[SB];     // rgb (xyz)
+};
+
+// The trilinear interpolant of 8 corner densities as a polynomial in the
+// place (x, y, z) in the unit cube: (1, z, y, yz) then (x, xz, xy, xyz).  Seven
+// multiply-adds evaluate it (trilinear_poly), against fifteen multiplies for
+// the corner weights and eight multiply-adds over them; 12 subtractions per
+// staged record set it up.
+__device__ __forceinline__ void trilinear_coefficients(const float g[8], float4& lo, float4& hi) {
+  const float z0 = g[1] - g[0], z1 = g[3] - g[2], z2 = g[5] - g[4], z3 = g[7] - g[6];
+  lo = make_float4(g[0], z0, g[2] - g[0], z1 - z0);
+  hi = make_float4(g[4] - g[0], z2 - z0, (g[6] - g[4]) - (g[2] - g[0]), (z3 - z2) - (z1 - z0));
+}
+__device__ __forceinline__ float trilinear_poly(const float4& lo, const float4& hi, float qx, float qy, float qz) {
+  const float a = fmaf(lo.y, qz, lo.x), b = fmaf(lo.w, qz, lo.z);
+  const float c = fmaf(hi.y, qz, hi.x), d = fmaf(hi.w, qz, hi.z);
+  return fmaf(fmaf(d, qy, c), qx, fmaf(b, qy, a));
+}
 
 // MAYBE_GRID = false compiles the grid-point read out (kernels instantiated
 // apart for the per-voxel densities).
-template <int SB, bool MAYBE_GRID = true>
-__device__ __forceinline__ void stage_record(StageSmem<SB>& s, int slot, uint32_t val, const VoxelArrays& va,
-                                             float ox, float oy, float oz) {
+template <bool MAYBE_GRID>
+__device__ __forceinline__ void read_densities(const VoxelArrays& va, uint32_t vid, float g[8]) {
+  if (MAYBE_GRID && va.key) {
+    const int64_t* k = va.key + 8 * (size_t)vid;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) g[c] = va.grid_bf16 ? __bfloat162float(va.grid_bf16[k[c]]) : va.grid[k[c]];
+  } else if (va.geos_bf16) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(va.geos_bf16 + 8 * (size_t)vid);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float2 f = __bfloat1622float2(h[c]);
+      g[2 * c] = f.x;
+      g[2 * c + 1] = f.y;
+    }
+  } else {
+    const float4* p = reinterpret_cast<const float4*>(va.geos + 8 * (size_t)vid);
+    const float4 a = p[0], b = p[1];
+    g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w;
+    g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;
+  }
+}
+
+template <bool FAST, bool MAYBE_GRID, int SB>
+__device__ __forceinline__ void stage_record(FwdStage<SB>& s, int slot, uint32_t val, const VoxelArrays& va, float ox,
+                                             float oy, float oz) {
   const uint32_t vid = val_vox_id(val);
   const uint2 bb = va.bboxes[vid];
   s.box[slot] = make_uint4(bb_xmin(bb), bb_xmax(bb) - bb_xmin(bb), bb_ymin(bb),
@@ -109,46 +163,187 @@ __device__ __forceinline__ void stage_record(StageSmem<SB>& s, int slot, uint32_
   const float* c = va.centers + 3 * (size_t)vid;
   const float cx = c[0], cy = c[1], cz = c[2], len = va.lengths[vid];
   const float rad = 0.5f * len;
-  const float dx = cx - ox, dy = cy - oy, dz = cz - oz;
-  s.slab_lo[slot] = make_float4(dx - rad, dy - rad, dz - rad, 1.f / len);
-  s.slab_hi[slot] = make_float4(dx + rad, dy + rad, dz + rad, len);
-  s.corner[slot] = make_float4(cx - 0.5f * len, cy - 0.5f * len, cz - 0.5f * len, __int_as_float((int)vid));
-  if (MAYBE_GRID && va.key) {
-    const int64_t* k = va.key + 8 * (size_t)vid;
-    float g[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) g[c] = va.grid_bf16 ? __bfloat162float(va.grid_bf16[k[c]]) : va.grid[k[c]];
+  s.rel[slot] = make_float4(cx - ox, cy - oy, cz - oz, rad);
+  s.corner[slot] = make_float4(cx - rad, cy - rad, cz - rad, 1.f / len);
+  float g[8];
+  read_densities<MAYBE_GRID>(va, vid, g);
+  if (FAST) {
+    trilinear_coefficients(g, s.geo[slot][0], s.geo[slot][1]);
+  } else {
     s.geo[slot][0] = make_float4(g[0], g[1], g[2], g[3]);
     s.geo[slot][1] = make_float4(g[4], g[5], g[6], g[7]);
-  } else if (va.geos_bf16) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(va.geos_bf16 + 8 * (size_t)vid);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-    const float2 g0 = __bfloat1622float2(h[0]), g1 = __bfloat1622float2(h[1]);
-    const float2 g2 = __bfloat1622float2(h[2]), g3 = __bfloat1622float2(h[3]);
-    s.geo[slot][0] = make_float4(g0.x, g0.y, g1.x, g1.y);
-    s.geo[slot][1] = make_float4(g2.x, g2.y, g3.x, g3.y);
+  }
+  const float* rgb = va.rgbs + 3 * (size_t)vid;
+  s.rgb[slot] = make_float4(rgb[0], rgb[1], rgb[2], __int_as_float((int)vid));
+}
+
+template <bool FAST, bool MAYBE_GRID, int SB>
+__device__ __forceinline__ void stage_record(BwdStage<SB>& s, int slot, uint32_t val, const VoxelArrays& va, float ox,
+                                             float oy, float oz) {
+  const uint32_t vid = val_vox_id(val), quad = val_quadrant(val);
+  const uint2 bb = va.bboxes[vid];
+  s.box[slot] = make_uint4(bb_xmin(bb), bb_xmax(bb) - bb_xmin(bb), bb_ymin(bb),
+                           (bb_ymax(bb) - bb_ymin(bb)) | (quad << 16));
+  const float* c = va.centers + 3 * (size_t)vid;
+  const float cx = c[0], cy = c[1], cz = c[2], len = va.lengths[vid];
+  const float rad = 0.5f * len;
+  const float sx = (quad & 4u) ? -rad : rad, sy = (quad & 2u) ? -rad : rad, sz = (quad & 1u) ? -rad : rad;
+  const float dx = cx - ox, dy = cy - oy, dz = cz - oz;
+  s.near[slot] = make_float4(dx - sx, dy - sy, dz - sz, 1.f / len);
+  s.far[slot] = make_float4(dx + sx, dy + sy, dz + sz, 0.f);
+  s.corner[slot] = make_float4(cx - rad, cy - rad, cz - rad, __int_as_float((int)vid));
+  float g[8];
+  read_densities<MAYBE_GRID>(va, vid, g);
+  if (FAST) {
+    trilinear_coefficients(g, s.geo[slot][0], s.geo[slot][1]);
   } else {
-    const float4* g = reinterpret_cast<const float4*>(va.geos + 8 * (size_t)vid);
-    s.geo[slot][0] = g[0];
-    s.geo[slot][1] = g[1];
+    s.geo[slot][0] = make_float4(g[0], g[1], g[2], g[3]);
+    s.geo[slot][1] = make_float4(g[4], g[5], g[6], g[7]);
   }
   const float* rgb = va.rgbs + 3 * (size_t)vid;
   s.rgb[slot] = make_float4(rgb[0], rgb[1], rgb[2], 0.f);
 }
 
-// Slab test from the staged per-record terms (auxiliary.h:240-253).
-__device__ __forceinline__ float2 staged_ray_box(const float4& lo, const float4& hi, const PixelRay& r) {
-  const float ax = lo.x * r.ix, ay = lo.y * r.iy, az = lo.z * r.iz;
-  const float bx = hi.x * r.ix, by = hi.y * r.iy, bz = hi.z * r.iz;
-  const float nx = fminf(ax, bx), ny = fminf(ay, by), nz = fminf(az, bz);
-  const float fx = fmaxf(ax, bx), fy = fmaxf(ay, by), fz = fmaxf(az, bz);
-  return make_float2(fmaxf(fmaxf(nx, ny), nz), fminf(fminf(fx, fy), fz));
+// A plain CTA composites an 8x8 block but walks the list of the 16x16 tile
+// around it, most of whose records do not reach the block.  The list is read
+// NT entries at a time (value and bbox only, the next entries fetched while
+// the staged ones are composited); entries that reach the block wait in a ring
+// with their list positions until a round of them can be staged.
+template <class CFG>
+struct ListFilter {
+  uint2 ring[2 * CFG::NT];      // value, list position (from the walk's end of the list)
+  uint32_t hits[2][CFG::NW];    // per warp, alternating between chunks
+  uint32_t pos[CFG::SB];        // list positions of the staged records
+};
+
+// BACK: entries from the end of the range.  All members are uniform over the
+// CTA but the fetched entry.
+template <class CFG, bool BACK>
+struct ListReader {
+  uint2 range;
+  int total, next, head, tail, flip;
+  uint32_t bx0, by0;
+  uint32_t val;
+  uint2 bb;
+  bool got;
+
+  __device__ __forceinline__ void fetch(const uint32_t* __restrict__ vals, const VoxelArrays& va) {
+    const int i = next + (int)threadIdx.x;
+    got = i < total;
+    if (got) {
+      val = vals[BACK ? range.y - 1 - i : range.x + i];
+      bb = va.bboxes[val_vox_id(val)];
+    }
+  }
+  __device__ __forceinline__ void init(uint2 r, int tile_x, int tile_y, const uint32_t* __restrict__ vals,
+                                       const VoxelArrays& va) {
+    range = r;
+    total = (int)(r.y - r.x);
+    next = head = tail = flip = 0;
+    bx0 = tile_x * CFG::TS;
+    by0 = tile_y * CFG::TS;
+    fetch(vals, va);
+  }
+  // Next round of records (0: the list is through), left in ring entries
+  // [head - n, head).  Called by the whole CTA.
+  __device__ __forceinline__ int round(ListFilter<CFG>& f, const uint32_t* __restrict__ vals, const VoxelArrays& va) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    while (tail - head < CFG::SB && next < total) {
+      const bool hit = got && bb_xmin(bb) <= bx0 + (CFG::TS - 1) && bb_xmax(bb) >= bx0 &&
+                       bb_ymin(bb) <= by0 + (CFG::TS - 1) && bb_ymax(bb) >= by0;
+      const uint32_t m = __ballot_sync(0xffffffffu, hit);
+      if (lane == 0) f.hits[flip][warp] = __popc(m);
+      const uint32_t v = val;
+      const int i = next + (int)threadIdx.x;
+      next += CFG::NT;
+      fetch(vals, va);
+      __syncthreads();
+      int at = tail;
+#pragma unroll
+      for (int w = 0; w < CFG::NW; ++w) {
+        const int c = (int)f.hits[flip][w];
+        if (w < warp) at += c;
+        tail += c;
+      }
+      if (hit) f.ring[(at + __popc(m & lanemask_lt())) & (2 * CFG::NT - 1)] = make_uint2(v, (uint32_t)i);
+      flip ^= 1;
+    }
+    __syncthreads();
+    const int n = min(CFG::SB, tail - head);
+    head += n;
+    return n;
+  }
+  __device__ __forceinline__ uint2 entry(const ListFilter<CFG>& f, int n, int i) const {
+    return f.ring[(head - n + i) & (2 * CFG::NT - 1)];
+  }
+};
+
+// Slab test (auxiliary.h:240-253) of a ray of the record's octant: the octant
+// says which plane of each slab comes first, so no minima of the two are
+// needed.  A ray in a slab's plane (0 * inf) gives NaN, which fails a <= b: it
+// misses, as with the minima.
+__device__ __forceinline__ float2 octant_ray_box(const float4& rel, const PixelRay& r) {
+  const float sx = (r.quad & 4u) ? -rel.w : rel.w, sy = (r.quad & 2u) ? -rel.w : rel.w,
+              sz = (r.quad & 1u) ? -rel.w : rel.w;
+  return make_float2(max3_nan((rel.x - sx) * r.ix, (rel.y - sy) * r.iy, (rel.z - sz) * r.iz),
+                     min3_nan((rel.x + sx) * r.ix, (rel.y + sy) * r.iy, (rel.z + sz) * r.iz));
+}
+
+// The same from the two planes staged in crossing order.
+__device__ __forceinline__ float2 near_far_ray_box(const float4& nr, const float4& fr, const PixelRay& r) {
+  return make_float2(max3_nan(nr.x * r.ix, nr.y * r.iy, nr.z * r.iz),
+                     min3_nan(fr.x * r.ix, fr.y * r.iy, fr.z * r.iz));
+}
+
+// Fast arithmetic: exp(-optical depth) of a segment from its samples' summed
+// activations.  The backward divides T by 1 - alpha, which for an opaque voxel
+// keeps few digits: it has to arrive at the forward's alpha bit for bit, so both
+// call this.
+__device__ __forceinline__ float fast_transmittance(float step_sz, float act_sum) {
+  return ex2_approx((-kStepScale * kLog2E * step_sz) * act_sum);
+}
+
+// Transmittance exp(-optical depth) of the ray segment [a, b] through staged
+// record j (forward.cu:228-248): midpoint samples of the activated trilinear
+// density.  local_alpha (or nullptr) receives each sample's own opacity.
+template <int NS, bool FAST, int SB>
+__device__ __forceinline__ float record_transmittance(const FwdStage<SB>& s, int j, const PixelRay& ray, float a,
+                                                      float b, float* local_alpha) {
+  const float4 cr = s.corner[j], glo = s.geo[j][0], ghi = s.geo[j][1];
+  float vol_int = 0.f;
+  const float vox_l_inv = cr.w;
+  const float step_sz = (b - a) * (1.f / NS);
+  const float stx = step_sz * ray.dx, sty = step_sz * ray.dy, stz = step_sz * ray.dz;
+  const float t0 = a + 0.5f * step_sz;
+  const float ptx = ray.ox + t0 * ray.dx, pty = ray.oy + t0 * ray.dy, ptz = ray.oz + t0 * ray.dz;
+  float qx = (ptx - cr.x) * vox_l_inv;
+  float qy = (pty - cr.y) * vox_l_inv;
+  float qz = (ptz - cr.z) * vox_l_inv;
+  const float qsx = stx * vox_l_inv, qsy = sty * vox_l_inv, qsz = stz * vox_l_inv;
+#pragma unroll
+  for (int k = 0; k < NS; ++k) {
+    if (FAST) {
+      vol_int += density_act_f<true>(trilinear_poly(glo, ghi, qx, qy, qz));
+    } else {
+      const float geo[8] = {glo.x, glo.y, glo.z, glo.w, ghi.x, ghi.y, ghi.z, ghi.w};
+      float w[8];
+      trilinear_weights(qx, qy, qz, w);
+      float d = 0.f;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) d += geo[c] * w[c];
+      const float lvi = kStepScale * step_sz * density_act(d);
+      vol_int += lvi;
+      if (local_alpha) local_alpha[k] = fminf(kMaxAlpha, 1.f - expf(-lvi));
+    }
+    qx = qx + qsx; qy = qy + qsy; qz = qz + qsz;
+  }
+  return FAST ? fast_transmittance(step_sz, vol_int) : expf(-vol_int);
 }
 
 // Does staged record `slot` possibly touch a pixel of this warp's 8x4
 // micro-tile with a matching ray quadrant?
-template <int SB>
-__device__ __forceinline__ bool record_hits_warp(const StageSmem<SB>& s, int slot, uint32_t wx0, uint32_t wy0,
+template <class STAGE>
+__device__ __forceinline__ bool record_hits_warp(const STAGE& s, int slot, uint32_t wx0, uint32_t wy0,
                                                  uint32_t quad_mask) {
   const uint4 b = s.box[slot];
   return b.x <= wx0 + 7u && b.x + b.y >= wx0 && b.z <= wy0 + 3u && b.z + (b.w & 0xFFFFu) >= wy0 &&
@@ -187,15 +382,15 @@ __device__ __forceinline__ uint32_t block_cover_mask(const uint4& b, uint32_t bx
 // The reference's per-pixel test: pixel inside the packed bbox and ray
 // quadrant equal to the instance's (forward.cu:186), as two unsigned range
 // checks on the staged (min, extent) form.
-template <int SB>
-__device__ __forceinline__ bool record_hits_pixel(const StageSmem<SB>& s, int j, uint32_t px, uint32_t py,
+template <class STAGE>
+__device__ __forceinline__ bool record_hits_pixel(const STAGE& s, int j, uint32_t px, uint32_t py,
                                                   uint32_t quad) {
   const uint4 b = s.box[j];
   return (px - b.x) <= b.y && (py - b.z) <= (b.w & 0xFFFFu) && (b.w >> 16) == quad;
 }
 
-template <int SB>
-__device__ __forceinline__ void load_geo(const StageSmem<SB>& s, int j, float g[8]) {
+template <class STAGE>
+__device__ __forceinline__ void load_geo(const STAGE& s, int j, float g[8]) {
   const float4 a = s.geo[j][0], b = s.geo[j][1];
   g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w;
   g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;

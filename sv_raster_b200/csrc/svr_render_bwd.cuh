@@ -7,10 +7,10 @@
 // (:295-323), T recovery (:333), colour / distortion / normal / depth /
 // ascending / colour-concentration terms (:344-510) and the 12-float
 // gradient pack (:515-522).  The reference issues 12 global atomics per
-// contributing (pixel, voxel); here each warp reduces its lanes' gradients
-// with shuffles into a shared-memory accumulator per staged record
-// (GradAcc), and each record is flushed once per tile (16-byte vector
-// reductions where the gradient rows are aligned).
+// contributing (pixel, voxel); here a warp's lanes write their gradients as rows
+// into shared memory (GradRows), each record's rows are summed, and a record is
+// flushed once per warp (16-byte vector reductions where the gradient rows are
+// aligned).
 #pragma once
 
 #include "svr_render.cuh"
@@ -27,9 +27,6 @@ struct BwdTileIn {
   const float* gt_color;   // [3,H,W] or nullptr
   const float* out_depth;  // [3,H,W] or nullptr (distortion prefix sums)
   float lambda_R_concen, lambda_ascending, lambda_dist;
-  // A record's gradients from at most this many lanes go straight into its
-  // shared accumulator with atomics; more lanes use the warp reduce-scatter.
-  int atomic_lanes;
 };
 
 struct BwdTileOut {
@@ -44,186 +41,91 @@ struct BwdTileOut {
   float* grid_grad = nullptr;
 };
 
-// Density part of one record's flush: its 8 corner gradients into the
-// voxel's dL_dgeos row (two 16-byte reductions where the rows are aligned),
-// or into the grid points its corners index.
-template <bool MAYBE_GRID = true>
-__device__ __forceinline__ void flush_density(const BwdTileOut& out, uint32_t vid, const float acc[12], bool vec4) {
-  if (MAYBE_GRID && out.key) {
-    const int64_t* k = out.key + 8 * (size_t)vid;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) atomicAdd(out.grid_grad + k[c], acc[c]);
-    return;
-  }
-  float* g = out.dL_dgeos + 8 * (size_t)vid;
-  if (vec4) {
-    atomicAdd(reinterpret_cast<float4*>(g), make_float4(acc[0], acc[1], acc[2], acc[3]));
-    atomicAdd(reinterpret_cast<float4*>(g) + 1, make_float4(acc[4], acc[5], acc[6], acc[7]));
-  } else {
-#pragma unroll
-    for (int c = 0; c < 8; ++c) atomicAdd(g + c, acc[c]);
-  }
-}
-
-constexpr int kGradStride = 13;  // 12 gradient floats + 1 pad (bank spread)
-
-__device__ __forceinline__ float warp_sum(float x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
-}
-
-// Reduce-scatter of 12 per-lane values over the warp in 13 shuffles: halve
-// 12 -> 6 (xor 16) -> 3 (xor 8), pad the 3 to 4 and halve 4 -> 2 (xor 4)
-// -> 1 (xor 2), then add the pair (xor 1).  Lane l ends holding in v[0] the
-// warp total of slot 6*b4 + 3*b3 + 2*b2 + b1 (b_i = bit i of l) when
-// 2*b2 + b1 < 3; returns that slot for the even lane that should publish it
-// (-1 otherwise or for the padding slot).  Every slot 0-11 is published by
-// exactly one lane.
-__device__ __forceinline__ int warp_reduce_scatter12(float v[12], int lane) {
-  // step 1 (xor 16): keep slots 0-5 (bit 4 clear) or 6-11 (bit 4 set)
-  float a[6];
-  const bool hi16 = lane & 16;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const float send = hi16 ? v[k] : v[k + 6];
-    const float keep = hi16 ? v[k + 6] : v[k];
-    a[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-  }
-  // step 2 (xor 8): keep 3 of 6
-  float b[3];
-  const bool hi8 = lane & 8;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float send = hi8 ? a[k] : a[k + 3];
-    const float keep = hi8 ? a[k + 3] : a[k];
-    b[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-  }
-  // step 3 (xor 4): the 3 padded to 4, keep 2 (bit 2 set: slot 2 and the pad)
-  const bool hi4 = lane & 4;
-  const float c0 = (hi4 ? b[2] : b[0]) + __shfl_xor_sync(0xffffffffu, hi4 ? b[0] : b[2], 4);
-  const float c1 = (hi4 ? 0.f : b[1]) + __shfl_xor_sync(0xffffffffu, hi4 ? b[1] : 0.f, 4);
-  // step 4 (xor 2): keep 1 of 2
-  const bool hi2 = lane & 2;
-  float d = (hi2 ? c1 : c0) + __shfl_xor_sync(0xffffffffu, hi2 ? c0 : c1, 2);
-  // step 5 (xor 1): full sum on both lanes of the pair
-  d += __shfl_xor_sync(0xffffffffu, d, 1);
-  v[0] = d;
-  const int local = (hi4 ? 2 : 0) + (hi2 ? 1 : 0);
-  return ((lane & 1) == 0 && local < 3) ? (hi16 ? 6 : 0) + (hi8 ? 3 : 0) + local : -1;
-}
-
-// FAST selects the arithmetic of the per-(pixel, voxel) loop (exp_f, div_f in
-// svr_common.cuh); RGB4 the [P,4] colour-gradient layout whose rows, like the
-// density rows, are flushed with one 16-byte vector reduction each.
-// Per-record gradient accumulators of one staging round.  With at most two
-// warps per CTA and 32 records staged per round, each warp owns a slot per
-// staged record: a warp visits a record at most once per round, so the
-// record's warp total is stored with plain stores, a bitmask per 32-record
-// group marks the slots written this round, and the flush adds the (at most
-// two) slots -- no shared-memory atomics and no zeroing.  Other
-// configurations share one slot per record and add into it with
-// shared-memory atomics (per-warp slots for 64 records would cost the 64-
-// thread CTAs their 16th resident CTA per SM: measured slower).
-//
-// A record reached by few lanes (2 to kFewLanes, a third of the records a
-// warp contributes to at 1080p over the c4 scene) is summed by transposing
-// through a small per-warp area instead of the 13-shuffle reduce-scatter:
-// each contributing lane stores its 12 values as one row, then lanes 0-11
-// each add one column over the rows.
-template <class CFG>
-struct GradAcc {
-  static constexpr bool kPerWarp = CFG::NW <= 2 && CFG::SB <= 32;
-  static constexpr int kStride = kPerWarp ? 12 : kGradStride;  // 48-byte rows: 16-byte vector access
-  static constexpr int kFewLanes = 8;
-  static constexpr int kSlots = (kPerWarp ? CFG::NW : 1) * CFG::SB * kStride;
-  // accumulators, then the transposition rows (16-byte aligned)
-  static constexpr int kRowsAt = (kSlots + 3) / 4 * 4;
-  static constexpr int kFloats = kRowsAt + CFG::NW * kFewLanes * 12;
-  static constexpr int kWords = kPerWarp ? CFG::NW * CFG::GROUPS : 1;
-
-  __device__ static void init(float* s_grad, int tid) {
-    if (!kPerWarp)
-      for (int i = tid; i < CFG::SB * kStride; i += CFG::NT) s_grad[i] = 0.f;
-  }
-
-  // The warp's gradients of staged record j (gp: this lane's 12 values,
-  // meaningful where `contrib`; act_mask: the contributing lanes).
-  __device__ static void add(float* s_grad, int warp, int j, float gp[12], int lane, uint32_t act_mask,
-                             bool contrib, int atomic_lanes) {
-    const int k = __popc(act_mask);
-    float* acc = s_grad + ((kPerWarp ? warp * CFG::SB : 0) + j) * kStride;
-    if (kPerWarp ? k == 1 : k <= atomic_lanes) {
-      if (contrib) {  // one (or, shared slots, a few) lane(s): their values go straight in
-        if (kPerWarp) store_row(acc, gp);
-        else
-#pragma unroll
-          for (int c = 0; c < 12; ++c) atomicAdd(acc + c, gp[c]);
-      }
-    } else if (k <= kFewLanes) {
-      float* rows = s_grad + kRowsAt + warp * kFewLanes * 12;
-      if (contrib) store_row(rows + 12 * __popc(act_mask & ((1u << lane) - 1u)), gp);
-      __syncwarp();
-      if (lane < 12) {
-        float sum = rows[lane];
-        for (int r = 1; r < k; ++r) sum += rows[12 * r + lane];
-        if (kPerWarp) acc[lane] = sum;
-        else atomicAdd(acc + lane, sum);
-      }
-      __syncwarp();  // the rows are reused by the warp's next record
+// Four of a record's 12 summed gradients to global memory: q = 0, 1 the
+// corner densities 4q .. 4q + 3 (a row of dL_dgeos, as one 16-byte reduction
+// where the rows are aligned, or the grid points that the corners index), q = 2
+// the colour and the subdivision priority.
+template <bool RGB4, bool MAYBE_GRID>
+__device__ __forceinline__ void flush_quad(const BwdTileOut& out, uint32_t vid, int q, const float4& v) {
+  if (v.x == 0.f && v.y == 0.f && v.z == 0.f && v.w == 0.f) return;
+  if (q == 2) {
+    if (RGB4) {
+      atomicAdd(reinterpret_cast<float4*>(out.dL_drgbs) + vid, v);
     } else {
-      if (!contrib) {
-#pragma unroll
-        for (int c = 0; c < 12; ++c) gp[c] = 0.f;
-      }
-      const int slot = warp_reduce_scatter12(gp, lane);
-      if (slot >= 0) {
-        if (kPerWarp) acc[slot] = gp[0];
-        else atomicAdd(acc + slot, gp[0]);
-      }
+      float* c = out.dL_drgbs + 3 * (size_t)vid;
+      atomicAdd(c, v.x);
+      atomicAdd(c + 1, v.y);
+      atomicAdd(c + 2, v.z);
+      atomicAdd(out.subdiv + vid, v.w);
+    }
+  } else if (MAYBE_GRID && out.key) {
+    const int64_t* k = out.key + 8 * (size_t)vid + 4 * q;
+    atomicAdd(out.grid_grad + k[0], v.x);
+    atomicAdd(out.grid_grad + k[1], v.y);
+    atomicAdd(out.grid_grad + k[2], v.z);
+    atomicAdd(out.grid_grad + k[3], v.w);
+  } else {
+    float* g = out.dL_dgeos + 8 * (size_t)vid + 4 * q;
+    if (RGB4 || out.geo_vec4) {
+      atomicAdd(reinterpret_cast<float4*>(g), v);
+    } else {
+      atomicAdd(g, v.x);
+      atomicAdd(g + 1, v.y);
+      atomicAdd(g + 2, v.z);
+      atomicAdd(g + 3, v.w);
     }
   }
+}
 
-  __device__ static void store_row(float* row, const float gp[12]) {
-    float4* a4 = reinterpret_cast<float4*>(row);
-    a4[0] = make_float4(gp[0], gp[1], gp[2], gp[3]);
-    a4[1] = make_float4(gp[4], gp[5], gp[6], gp[7]);
-    a4[2] = make_float4(gp[8], gp[9], gp[10], gp[11]);
-  }
-
-  // End of group g of a warp's hit loop: `wrote` marks the records it stored.
-  __device__ static void mark(uint32_t* s_hit, int warp, int g, uint32_t wrote, int lane) {
-    if (kPerWarp && lane == 0) s_hit[warp * CFG::GROUPS + g] = wrote;
-  }
-
-  // Record t's total over the CTA this round; false when no warp wrote it.
-  __device__ static bool gather(float* s_grad, const uint32_t* s_hit, int t, float a[12]) {
-    if (kPerWarp) {
-      bool any = false;
-#pragma unroll
-      for (int c = 0; c < 12; ++c) a[c] = 0.f;
-#pragma unroll
-      for (int w = 0; w < CFG::NW; ++w) {
-        if (!((s_hit[w * CFG::GROUPS + (t >> 5)] >> (t & 31)) & 1u)) continue;
-        any = true;
-        const float4* a4 = reinterpret_cast<const float4*>(s_grad + (w * CFG::SB + t) * kStride);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          const float4 v = a4[q];
-          a[4 * q] += v.x; a[4 * q + 1] += v.y; a[4 * q + 2] += v.z; a[4 * q + 3] += v.w;
-        }
-      }
-      return any;
-    }
-    float* acc = s_grad + t * kStride;
-#pragma unroll
-    for (int c = 0; c < 12; ++c) {
-      a[c] = acc[c];
-      acc[c] = 0.f;
-    }
-    return true;
-  }
+// Gradient rows of one warp.  Every (record, pixel) pair of a run of records
+// has a row of 12 values (8 corner densities, 3 colour, 1 subdivision
+// priority), a record's rows next to each other in pixel order; the lanes
+// fill them while each walks its own pixel's records, then add them up
+// record by record.  64 rows (3.6 KB a warp): 128 leave the staging's gathers
+// less of the L1 cache, 40 cut the runs too short (5.7 / 6.4 / 6.3 ms for 64 /
+// 128 / 40 with 16 views of 2M voxels).
+template <int ROWS_>
+struct GradRows {
+  static constexpr int kRows = ROWS_;
+  static_assert(ROWS_ >= 32, "a record may take a row per lane");
+  float4 row[ROWS_][3];
+  uint2 pairs[32];  // by record of the group: lanes that take it, its first row
+  uint2 recs[32];   // by place in the run: voxel id, first row | rows << 16
 };
+template <class CFG>
+using TileRows = GradRows<64>;
+
+// Sums the rows of the run's n_rec records and sends them off.  Lanes take
+// (record, four of its values) and, while lanes are left over, a half or a
+// quarter of its rows.
+template <bool RGB4, bool MAYBE_GRID, class ROWS>
+__device__ __forceinline__ void flush_rows(const ROWS& g, int n_rec, int lane, const BwdTileOut& out) {
+  __syncwarp();
+  const int fs = n_rec <= 2 ? 2 : (n_rec <= 5 ? 1 : 0);  // log2 of the lanes per (record, values)
+  const int n = (3 * n_rec) << fs;
+  for (int e0 = 0; e0 < n; e0 += 32) {
+    const int e = e0 + lane;
+    const int rq = min(e, n - 1) >> fs;
+    const int r = rq / 3, q = rq - 3 * r;
+    const uint2 rec = g.recs[r];
+    const int i0 = (int)(rec.y & 0xFFFFu), i1 = i0 + (int)(rec.y >> 16);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = i0 + (e & ((1 << fs) - 1)); i < i1; i += 1 << fs) {
+      const float4 x = g.row[i][q];
+      v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+    }
+    __syncwarp();
+    for (int d = 1; d < (1 << fs); d <<= 1) {
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, d);
+      v.y += __shfl_xor_sync(0xffffffffu, v.y, d);
+      v.z += __shfl_xor_sync(0xffffffffu, v.z, d);
+      v.w += __shfl_xor_sync(0xffffffffu, v.w, d);
+    }
+    if (e < n && (e & ((1 << fs) - 1)) == 0)
+      flush_quad<RGB4, MAYBE_GRID>(out, rec.x, q, v);
+  }
+  __syncwarp();
+}
 
 // Per-pixel state of the backward walk (the pixel's upstream gradients, its
 // transmittance being recovered record by record, and the running sums).
@@ -280,7 +182,7 @@ __device__ __forceinline__ BwdPix bwd_pixel_init(const ViewParams& vp, const Bwd
 // colour, 1 subdivision priority) in gp.  Returns whether the record
 // contributes (gp is left unset otherwise).
 template <int SB, int NS, bool DEPTH, bool DIST, bool NORMAL, bool FAST>
-__device__ __forceinline__ bool bwd_pixel_record(const StageSmem<SB>& s, int j, const PixelRay& ray,
+__device__ __forceinline__ bool bwd_pixel_record(const FwdStage<SB>& s, int j, const PixelRay& ray,
                                                  const BwdTileIn& in, BwdPix& st, float gp[12]) {
   float& T = st.T;
   float& last_dL_dT = st.last_dL_dT;
@@ -294,15 +196,14 @@ __device__ __forceinline__ bool bwd_pixel_record(const StageSmem<SB>& s, int j, 
   (void)dL_dD; (void)dNx; (void)dNy; (void)dNz; (void)weight_dist;
   (void)prefix_wm; (void)suffix_wm; (void)prefix_w; (void)suffix_w;
   bool contrib = false;
-  // Fast arithmetic, one sample, no depth terms: keep the trilinear weights
-  // and scale them once by dL/dI * d(density)/d(sample) (8 multiplies fewer
-  // than forming dI/dgeo first; a different rounding order).
-  constexpr bool kFoldScale = FAST && NS == 1 && !DEPTH;
-  const float4 slo = s.slab_lo[j], shi = s.slab_hi[j];
-  const float2 ab = staged_ray_box(slo, shi, ray);
+  // One sample, no depth terms: dL/dgeo is dL/d(density) times the corner
+  // weights; the fast arithmetic splits it axis by axis instead of forming
+  // the weights (the density itself is a polynomial there).
+  constexpr bool kFoldScale = NS == 1 && !DEPTH;
+  const float2 ab = octant_ray_box(s.rel[j], ray);
   const float a = ab.x, b = ab.y;
-  if (!(a > b)) {
-    float geo[8];
+  {
+    float geo[8];  // with the fast arithmetic: the density polynomial
     load_geo(s, j, geo);
     float dgeo[8];
 #pragma unroll
@@ -314,8 +215,8 @@ __device__ __forceinline__ bool bwd_pixel_record(const StageSmem<SB>& s, int j, 
     float each_dI[NS][8];
     float w[8];
     float local_alpha[NS];
-    const float vox_l_inv = slo.w;
     const float4 cr = s.corner[j];
+    const float vox_l_inv = cr.w;
     const float step_sz = (b - a) * (1.f / NS);
     const float stx = step_sz * ray.dx, sty = step_sz * ray.dy, stz = step_sz * ray.dz;
     const float t0 = a + 0.5f * step_sz;
@@ -326,18 +227,23 @@ __device__ __forceinline__ bool bwd_pixel_record(const StageSmem<SB>& s, int j, 
     const float qsx = stx * vox_l_inv, qsy = sty * vox_l_inv, qsz = stz * vox_l_inv;
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
-      trilinear_weights(qx, qy, qz, w);
+      if (!(FAST && kFoldScale)) trilinear_weights(qx, qy, qz, w);
       float d = 0.f;
+      if (FAST) {
+        d = trilinear_poly(make_float4(geo[0], geo[1], geo[2], geo[3]), make_float4(geo[4], geo[5], geo[6], geo[7]),
+                           qx, qy, qz);
+      } else {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) d += geo[c] * w[c];
+        for (int c = 0; c < 8; ++c) d += geo[c] * w[c];
+      }
       float act, act_grad;
       density_act_and_grad_f<FAST>(d, act, act_grad);
       const float lvi = kStepScale * step_sz * act;
-      vol_int += lvi;
-      if (DEPTH && NS > 1) local_alpha[k] = fminf(kMaxAlpha, 1.f - exp_f<FAST>(-lvi));
+      vol_int += FAST ? act : lvi;
+      if (DEPTH && NS > 1) local_alpha[k] = fminf(kMaxAlpha, 1.f - expf(-lvi));
       const float dd_dd = kStepScale * step_sz * act_grad;
       if (kFoldScale) {
-        dI_dgeo[0] = dd_dd;  // the weights stay in w: dL/dgeo = (dL/dI * dd_dd) * w below
+        dI_dgeo[0] = dd_dd;
       } else {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -346,11 +252,11 @@ __device__ __forceinline__ bool bwd_pixel_record(const StageSmem<SB>& s, int j, 
           if (DEPTH && NS > 1) each_dI[k][c] = tmp;
         }
       }
-      qx = qx + qsx; qy = qy + qsy; qz = qz + qsz;
+      if (k + 1 < NS) { qx = qx + qsx; qy = qy + qsy; qz = qz + qsz; }
     }
-    const float exp_neg = exp_f<FAST>(-vol_int);
+    const float exp_neg = FAST ? fast_transmittance(step_sz, vol_int) : expf(-vol_int);
     const float alpha = fminf(kMaxAlpha, 1.f - exp_neg);
-    if (!(alpha < kMinAlpha)) {
+    if (a <= b && !(alpha < kMinAlpha)) {
       contrib = true;
       T = div_f<FAST>(T, 1.f - alpha);
       const float pt_w = alpha * T;
@@ -391,7 +297,16 @@ __device__ __forceinline__ bool bwd_pixel_record(const StageSmem<SB>& s, int j, 
       const float dL_dalpha = T * (dL_dpt_w - last_dL_dT);
       last_dL_dT += alpha * (dL_dpt_w - last_dL_dT);
       const float dL_dI = dL_dalpha * exp_neg;
-      if (kFoldScale) {
+      if (kFoldScale && FAST) {
+        const float s1 = dL_dI * dI_dgeo[0];
+        const float x1 = s1 * qx, x0 = s1 - x1;
+        const float x0y1 = x0 * qy, x0y0 = x0 - x0y1;
+        const float x1y1 = x1 * qy, x1y0 = x1 - x1y1;
+        dgeo[1] = x0y0 * qz; dgeo[0] = x0y0 - dgeo[1];
+        dgeo[3] = x0y1 * qz; dgeo[2] = x0y1 - dgeo[3];
+        dgeo[5] = x1y0 * qz; dgeo[4] = x1y0 - dgeo[5];
+        dgeo[7] = x1y1 * qz; dgeo[6] = x1y1 - dgeo[7];
+      } else if (kFoldScale) {
         const float sI = dL_dI * dI_dgeo[0];
 #pragma unroll
         for (int c = 0; c < 8; ++c) dgeo[c] += sI * w[c];
@@ -437,7 +352,7 @@ __device__ __forceinline__ bool bwd_pixel_record(const StageSmem<SB>& s, int j, 
           for (int c = 0; c < 8; ++c) dgeo[c] += dI[0] * dI_dgeo[c];
         }
       }
-      if (in.lambda_ascending > 0) {
+      if (!FAST && in.lambda_ascending > 0) {
         const float lo_x = cr.x, lo_y = cr.y, lo_z = cr.z;
         const float pax = ray.ox + a * ray.dx, pay = ray.oy + a * ray.dy, paz = ray.oz + a * ray.dz;
         const float pbx = ray.ox + b * ray.dx, pby = ray.oy + b * ray.dy, pbz = ray.oz + b * ray.dz;
@@ -470,14 +385,21 @@ __device__ __forceinline__ bool bwd_pixel_record(const StageSmem<SB>& s, int j, 
   return contrib;
 }
 
-template <class CFG, int NS, bool DEPTH, bool DIST, bool NORMAL, bool FAST = false, bool RGB4 = false>
+// One tile, one pixel per thread, each warp an 8x4 block of its own.  Each lane
+// walks its own pixel's records of a staged batch, as in the forward, so a warp
+// takes as many iterations as its busiest pixel has records and not one per
+// record that touches it; the 12 gradients of each pair go to the record's rows
+// (GradRows), which are summed when the run of records that they have room
+// for is through.  RGB4: the [P,4] colour-gradient layout, and 16-byte aligned
+// density rows.
+template <class CFG, int NS, bool DEPTH, bool DIST, bool NORMAL, bool FAST = false, bool RGB4 = false,
+          bool MAYBE_GRID = false, bool SHARED_LIST = false>
 __device__ __forceinline__ void render_tile_bwd(const ViewParams& vp, const float* __restrict__ c2w_s, int tile_x,
                                                 int tile_y, uint2 range_raw, uint32_t tile_last,
                                                 const uint32_t* __restrict__ vals, const VoxelArrays& va,
-                                                const BwdTileIn& in, const BwdTileOut& out, StageSmem<CFG::SB>& s,
-                                                float* s_grad /*[GradAcc::kFloats]*/,
-                                                uint32_t* s_hit /*[GradAcc::kWords]*/) {
-  using Acc = GradAcc<CFG>;
+                                                const BwdTileIn& in, const BwdTileOut& out, FwdStage<CFG::SB>& s,
+                                                TileRows<CFG>* s_rows /*[CFG::NW]*/,
+                                                ListFilter<CFG>* s_list = nullptr) {
   constexpr int SB = CFG::SB;
   const int W = vp.W, H = vp.H;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -486,9 +408,10 @@ __device__ __forceinline__ void render_tile_bwd(const ViewParams& vp, const floa
   const uint32_t px = tile_x * CFG::TS + lx, py = tile_y * CFG::TS + ly;
   const uint32_t pix_id = (uint32_t)W * py + px;
   const bool inside = px < (uint32_t)W && py < (uint32_t)H;
-  const PixelRay ray = make_pixel_ray((float)px, (float)py, W, H, vp.tanfovx, vp.tanfovy, vp.cx, vp.cy, c2w_s);
+  const PixelRay ray = make_pixel_ray<!RGB4>((float)px, (float)py, W, H, vp.tanfovx, vp.tanfovy, vp.cx, vp.cy, c2w_s);
   const int warp = tid >> 5;
   const uint32_t wx0 = tile_x * CFG::TS + (warp % CFG::MX) * 8, wy0 = tile_y * CFG::TS + (warp / CFG::MX) * 4;
+  TileRows<CFG>& rows = s_rows[warp];
 
   // Range check (replaces the __trap at backward.cu:122-133).
   if (tile_last > range_raw.y || range_raw.x > tile_last) {
@@ -502,7 +425,6 @@ __device__ __forceinline__ void render_tile_bwd(const ViewParams& vp, const floa
   const uint32_t last_contrib = inside ? in.n_contrib[pix_id] : 0u;
   BwdPix st = bwd_pixel_init<DEPTH, DIST, NORMAL>(vp, in, ray, inside, pix_id, T_final);
 
-  Acc::init(s_grad, tid);
   // Largest contributor count of this warp: records at or beyond it are skipped by every lane.
   const uint32_t warp_lc = __reduce_max_sync(0xffffffffu, last_contrib);
   const uint32_t quad_mask = __reduce_or_sync(0xffffffffu, inside ? (1u << ray.quad) : 0u);
@@ -515,20 +437,36 @@ __device__ __forceinline__ void render_tile_bwd(const ViewParams& vp, const floa
   }
 
   const int rounds = (todo_total + SB - 1) / SB;
-  for (int r = 0; r < rounds; ++r) {
+  ListReader<CFG, true> list;
+  if (SHARED_LIST) list.init(range, tile_x, tile_y, vals, va);
+  for (int r = 0; SHARED_LIST || r < rounds; ++r) {
     __syncthreads();
     const int base = r * SB;                     // records [base, base+n_here) from the back
-    const int n_here = min(SB, todo_total - base);
-    for (int i = tid; i < n_here; i += CFG::NT)
-      stage_record(s, i, vals[range.y - base - i - 1], va, ray.ox, ray.oy, ray.oz);
+    const int n_here = SHARED_LIST ? list.round(*s_list, vals, va) : min(SB, todo_total - base);
+    if (SHARED_LIST && n_here == 0) break;
+    for (int i = tid; i < (SHARED_LIST ? SB : n_here); i += CFG::NT) {
+      uint32_t val;
+      if (SHARED_LIST) {
+        // positions relative to range.x; 0 past the round, in reach of everyone and covering nothing
+        if (i >= n_here) {
+          s_list->pos[i] = 0u;
+          continue;
+        }
+        const uint2 e = list.entry(*s_list, n_here, i);
+        val = e.x;
+        s_list->pos[i] = (uint32_t)(todo_total - 1) - e.y;
+      } else {
+        val = vals[range.y - base - i - 1];
+      }
+      stage_record<FAST, MAYBE_GRID>(s, i, val, va, ray.ox, ray.oy, ray.oz);
+    }
     __syncthreads();
 
-    // Position (relative to range.x) of staged slot j is todo_total - base - j - 1.
+    // Position (relative to range.x) of staged slot j is todo_total - base - j - 1, or in s_list.
     for (int g = 0; g < CFG::GROUPS && g * 32 < n_here; ++g) {
       const int slot = g * 32 + lane;
-      const uint32_t pos = (uint32_t)(todo_total - base - slot - 1);
+      const uint32_t pos = SHARED_LIST ? s_list->pos[slot] : (uint32_t)(todo_total - base - slot - 1);
       const bool hit = slot < n_here && pos < warp_lc && record_hits_warp(s, slot, wx0, wy0, quad_mask);
-      uint32_t m = __ballot_sync(0xffffffffu, hit);
       // This lane's candidate records of the group (pixel in the record's
       // bbox, matching quadrant, record within the contributor count): lane
       // j's block mask of record j, transposed across the warp.
@@ -539,46 +477,65 @@ __device__ __forceinline__ void render_tile_bwd(const ViewParams& vp, const floa
         rec_quad = b.w >> 16;
       }
       uint32_t mine = warp_transpose_bits(covers & __shfl_sync(0xffffffffu, qlanes, (int)rec_quad), (uint32_t)lane);
-      {
+      if (SHARED_LIST) {
+        // the first slot whose position is below this pixel's contributor
+        // count (positions fall with the slot)
+        int first = 0;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+          if (s_list->pos[g * 32 + first + d - 1] >= last_contrib) first += d;
+        if (s_list->pos[g * 32 + first] >= last_contrib) ++first;
+        mine &= first >= 32 ? 0u : ~((1u << first) - 1u);
+      } else {
         // slot j is in reach while todo_total - base - j - 1 < last_contrib
         const int first = todo_total - base - (int)last_contrib - g * 32;
         mine &= first <= 0 ? 0xffffffffu : (first >= 32 ? 0u : ~((1u << first) - 1u));
       }
-      m &= __reduce_or_sync(0xffffffffu, mine);  // records no pixel of the warp takes
-      uint32_t wrote = 0u;
-      while (m) {
-        const int bit = __ffs(m) - 1;
-        const int j = g * 32 + bit;
-        m &= m - 1;
-        bool contrib = false;
-        float gp[12];
-        if ((mine >> bit) & 1u) contrib = bwd_pixel_record<SB, NS, DEPTH, DIST, NORMAL, FAST>(s, j, ray, in, st, gp);
-        // Warp reduction of this record's gradients into its accumulator.
-        const uint32_t act_mask = __ballot_sync(0xffffffffu, contrib);
-        if (act_mask == 0u) continue;
-        Acc::add(s_grad, warp, j, gp, lane, act_mask, contrib, in.atomic_lanes);
-        wrote |= 1u << (j & 31);
+      // Back: lane j holds the lanes that take record j, and the records'
+      // rows one after the other.
+      const uint32_t takers = warp_transpose_bits(mine, (uint32_t)lane);
+      const uint32_t n_takers = __popc(takers);
+      uint32_t incl = n_takers;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += t;
       }
-      Acc::mark(s_hit, warp, g, wrote, lane);
-    }
-    __syncthreads();
-    // Flush this batch's accumulators: one set of reductions per (voxel, tile).
-    for (int t = tid; t < n_here; t += CFG::NT) {
-      float acc[12];
-      if (!Acc::gather(s_grad, s_hit, t, acc)) continue;
-      float gsum = 0.f;
-#pragma unroll
-      for (int c = 0; c < 12; ++c) gsum += fabsf(acc[c]);
-      if (gsum != 0.f) {
-        const uint32_t vid = (uint32_t)__float_as_int(s.corner[t].w);
-        flush_density(out, vid, acc, RGB4 || out.geo_vec4);
-        if (RGB4) {
-          atomicAdd(reinterpret_cast<float4*>(out.dL_drgbs) + vid, make_float4(acc[8], acc[9], acc[10], acc[11]));
-        } else {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) atomicAdd(out.dL_drgbs + 3 * (size_t)vid + c, acc[8 + c]);
-          atomicAdd(out.subdiv + vid, acc[11]);
+      mine = __brev(mine);  // record j of the group is bit 31 - j: walked highest bit first
+      uint32_t done_rows = 0u;
+      const uint32_t all_rows = __shfl_sync(0xffffffffu, incl, 31);
+      uint32_t left = 0xffffffffu;  // records not yet walked (bit j)
+      while (done_rows < all_rows) {
+        // the run of records whose rows fit
+        const bool in_run = ((left >> lane) & 1u) && incl - done_rows <= (uint32_t)TileRows<CFG>::kRows;
+        const uint32_t run = __ballot_sync(0xffffffffu, in_run);
+        const uint32_t used = __ballot_sync(0xffffffffu, in_run && n_takers > 0u);
+        const uint32_t first_row = incl - n_takers - done_rows;
+        if (in_run) {
+          rows.pairs[lane] = make_uint2(takers, first_row);
+          if (n_takers > 0u)
+            rows.recs[__popc(used & lanemask_lt())] = make_uint2((uint32_t)__float_as_int(s.rgb[slot].w), first_row | (n_takers << 16));
         }
+        done_rows = __shfl_sync(0xffffffffu, incl, 31 - __clz((int)run));
+        left &= ~run;
+        __syncwarp();
+        uint32_t walk = mine & __brev(run);
+        while (walk) {
+          const int bit = bfind(walk);
+          walk ^= 1u << bit;
+          const int jj = 31 - bit;
+          float gp[12];
+          if (!bwd_pixel_record<SB, NS, DEPTH, DIST, NORMAL, FAST>(s, g * 32 + jj, ray, in, st, gp)) {
+#pragma unroll
+            for (int c = 0; c < 12; ++c) gp[c] = 0.f;
+          }
+          const uint2 pr = rows.pairs[jj];
+          float4* row = rows.row[pr.y + __popc(pr.x & lanemask_lt())];
+          row[0] = make_float4(gp[0], gp[1], gp[2], gp[3]);
+          row[1] = make_float4(gp[4], gp[5], gp[6], gp[7]);
+          row[2] = make_float4(gp[8], gp[9], gp[10], gp[11]);
+        }
+        flush_rows<RGB4, MAYBE_GRID>(rows, __popc(used), lane, out);
       }
     }
   }

@@ -10,10 +10,16 @@
 
 namespace svr {
 
-int persistent_grid(const void* kernel, int threads, size_t dyn_smem, int n_items, int ctas_per_sm) {
-  int dev = 0, sms = 1, per_sm = 0;
+int sm_count() {
+  int dev = 0, n = 0;
   cudaGetDevice(&dev);
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n > 0 ? n : 148;
+}
+
+int persistent_grid(const void* kernel, int threads, size_t dyn_smem, int n_items, int ctas_per_sm) {
+  const int sms = sm_count();
+  int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, dyn_smem) != cudaSuccess ||
       per_sm < 1)
     per_sm = 1;
@@ -36,9 +42,10 @@ struct FwdArgs {
 template <int NS, bool DEPTH, bool DIST, bool NORMAL, bool MAXW>
 __global__ void __launch_bounds__(PlainTile::NT, fwd_min_blocks<PlainTile>())
 render_fwd_kernel(const __grid_constant__ FwdArgs a) {
-  __shared__ StageSmem<PlainTile::SB> s;
+  __shared__ FwdStage<PlainTile::SB> s;
   __shared__ float s_c2w[12];
   __shared__ uint32_t s_red[PlainTile::NW];
+  __shared__ ListFilter<PlainTile> s_list;
   if (threadIdx.x < 12) s_c2w[threadIdx.x] = a.vp.c2w[threadIdx.x];
   __syncthreads();
   const int b = blockIdx.x / kPlainSub, sub = blockIdx.x % kPlainSub;
@@ -46,7 +53,7 @@ render_fwd_kernel(const __grid_constant__ FwdArgs a) {
   const int tile_x = (tile % a.vp.grid_x) * 2 + (sub & 1), tile_y = (tile / a.vp.grid_x) * 2 + (sub >> 1);
   const uint2 range = a.ranges[tile];
   render_tile_fwd<PlainTile, NS, DEPTH, DIST, NORMAL, MAXW, true>(a.vp, s_c2w, tile_x, tile_y, range, a.vals, a.va,
-                                                                  a.out, a.out.tile_last + tile, s, s_red);
+                                                                  a.out, a.out.tile_last + tile, s, s_red, &s_list);
 }
 
 // Multi-view form: a persistent grid over the (view, tile) work items of all
@@ -70,7 +77,7 @@ struct FwdBatchArgs {
 
 template <class CFG>
 struct FwdBatchSmem {
-  StageSmem<CFG::SB> s;
+  FwdStage<CFG::SB> s;
   float c2w[12];
   uint32_t red[CFG::NW];
   uint32_t item;

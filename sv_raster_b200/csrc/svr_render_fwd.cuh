@@ -29,14 +29,15 @@ struct FwdTileOut {
 // (tile_x, tile_y) index CFG::TS-sized tiles; `range` is the list the tile
 // walks (its own, or the list of an enclosing tile it shares with others);
 // `last_slot` receives range.x + the tile's largest contributor count, with
-// atomicMax when SHARED_LAST (several CTAs share one list and slot, which
-// then starts at 0).
+// atomicMax when SHARED_LIST (several CTAs share one list, read through s_list,
+// and one slot, which then starts at 0).
 // FAST selects the arithmetic of the per-(pixel, voxel) loop (exp_f, svr_common.cuh).
-template <class CFG, int NS, bool DEPTH, bool DIST, bool NORMAL, bool MAXW, bool SHARED_LAST = false, bool FAST = false>
+template <class CFG, int NS, bool DEPTH, bool DIST, bool NORMAL, bool MAXW, bool SHARED_LIST = false, bool FAST = false>
 __device__ __forceinline__ void render_tile_fwd(const ViewParams& vp, const float* __restrict__ c2w_s, int tile_x,
                                                 int tile_y, uint2 range, const uint32_t* __restrict__ vals,
                                                 const VoxelArrays& va, const FwdTileOut& out, uint32_t* last_slot,
-                                                StageSmem<CFG::SB>& s, uint32_t* s_red /*[CFG::NW]*/) {
+                                                FwdStage<CFG::SB>& s, uint32_t* s_red /*[CFG::NW]*/,
+                                                ListFilter<CFG>* s_list = nullptr) {
   constexpr int SB = CFG::SB;
   const int W = vp.W, H = vp.H;
   const int tid = threadIdx.x;
@@ -60,13 +61,25 @@ __device__ __forceinline__ void render_tile_fwd(const ViewParams& vp, const floa
 
   const int todo_total = (int)(range.y - range.x);
   const int rounds = (todo_total + SB - 1) / SB;
-  for (int r = 0; r < rounds; ++r) {
+  ListReader<CFG, false> list;
+  if (SHARED_LIST) list.init(range, tile_x, tile_y, vals, va);
+  for (int r = 0; SHARED_LIST || r < rounds; ++r) {
     // All pixels finished: stop (also the barrier that frees the staging buffer).
     if (__syncthreads_count(done) == CFG::NT) break;
     const int base = r * SB;
-    const int n_here = min(SB, todo_total - base);
-    for (int i = tid; i < n_here; i += CFG::NT)
-      stage_record(s, i, vals[range.x + base + i], va, ray.ox, ray.oy, ray.oz);
+    const int n_here = SHARED_LIST ? list.round(*s_list, vals, va) : min(SB, todo_total - base);
+    if (SHARED_LIST && n_here == 0) break;
+    for (int i = tid; i < n_here; i += CFG::NT) {
+      uint32_t val;
+      if (SHARED_LIST) {
+        const uint2 e = list.entry(*s_list, n_here, i);
+        val = e.x;
+        s_list->pos[i] = e.y;
+      } else {
+        val = vals[range.x + base + i];
+      }
+      stage_record<FAST, true>(s, i, val, va, ray.ox, ray.oy, ray.oz);
+    }
     __syncthreads();
 
     const uint32_t quad_mask = __reduce_or_sync(0xffffffffu, done ? 0u : (1u << ray.quad));
@@ -101,46 +114,24 @@ __device__ __forceinline__ void render_tile_fwd(const ViewParams& vp, const floa
       // an earlier group of this round takes no more records.)
       uint32_t mine = warp_transpose_bits(covers, lane);
       if (done) mine = 0u;
+      // Highest bit first: record j of the group is bit 31 - j.
+      mine = __brev(mine);
       while (mine) {
-        const int j = g * 32 + __ffs(mine) - 1;
-        mine &= mine - 1;
-        const float4 slo = s.slab_lo[j], shi = s.slab_hi[j];
-        const float2 ab = staged_ray_box(slo, shi, ray);
+        const int bit = bfind(mine);
+        const int j = g * 32 + 31 - bit;
+        mine ^= 1u << bit;
+        // A ray that misses the cube (a > b, or NaN) runs through the density
+        // with the others: one branch per record instead of two.
+        const float2 ab = octant_ray_box(s.rel[j], ray);
         const float a = ab.x, b = ab.y;
-        if (a > b) continue;
-
-        float geo[8];
-        load_geo(s, j, geo);
-        float vol_int = 0.f;
-        float w[8];
         float local_alpha[NS];
-        const float vox_l_inv = slo.w;
-        const float4 cr = s.corner[j];
-        const float step_sz = (b - a) * (1.f / NS);
-        const float stx = step_sz * ray.dx, sty = step_sz * ray.dy, stz = step_sz * ray.dz;
-        const float t0 = a + 0.5f * step_sz;
-        const float ptx = ray.ox + t0 * ray.dx, pty = ray.oy + t0 * ray.dy, ptz = ray.oz + t0 * ray.dz;
-        float qx = (ptx - cr.x) * vox_l_inv;
-        float qy = (pty - cr.y) * vox_l_inv;
-        float qz = (ptz - cr.z) * vox_l_inv;
-        const float qsx = stx * vox_l_inv, qsy = sty * vox_l_inv, qsz = stz * vox_l_inv;
-#pragma unroll
-        for (int k = 0; k < NS; ++k) {
-          trilinear_weights(qx, qy, qz, w);
-          float d = 0.f;
-#pragma unroll
-          for (int c = 0; c < 8; ++c) d += geo[c] * w[c];
-          const float lvi = kStepScale * step_sz * density_act_f<FAST>(d);
-          vol_int += lvi;
-          if (DEPTH && NS > 1) local_alpha[k] = fminf(kMaxAlpha, 1.f - exp_f<FAST>(-lvi));
-          qx = qx + qsx; qy = qy + qsy; qz = qz + qsz;
-        }
-        const float alpha = fminf(kMaxAlpha, 1.f - exp_f<FAST>(-vol_int));
-        if (alpha < kMinAlpha) continue;
+        const float through = record_transmittance<NS, FAST>(s, j, ray, a, b, DEPTH && NS > 1 ? local_alpha : nullptr);
+        const float alpha = fminf(kMaxAlpha, 1.f - through);
+        if (!(a <= b) || alpha < kMinAlpha) continue;
 
         const float pt_w = T * alpha;
         const float4 rgbv = s.rgb[j];
-        const int vid = __float_as_int(cr.w);
+        const int vid = __float_as_int(rgbv.w);
         Cx = Cx + pt_w * rgbv.x;
         Cy = Cy + pt_w * rgbv.y;
         Cz = Cz + pt_w * rgbv.z;
@@ -167,6 +158,8 @@ __device__ __forceinline__ void render_tile_fwd(const ViewParams& vp, const floa
         }
         if (DIST) Ddist = Ddist + pt_w * 0.5f * (contract_depth(a) + contract_depth(b));
         if (NORMAL) {
+          float geo[8];
+          load_geo(s, j, geo);
           float nx, ny, nz;
           field_normal(geo, nx, ny, nz);
           const float rl = safe_rnorm3(nx, ny, nz);
@@ -175,7 +168,7 @@ __device__ __forceinline__ void render_tile_fwd(const ViewParams& vp, const floa
           Nz = Nz + pt_w * rl * nz;
         }
         T *= (1.f - alpha);
-        last_contrib = (uint32_t)(base + j + 1);
+        last_contrib = SHARED_LIST ? s_list->pos[j] + 1u : (uint32_t)(base + j + 1);
         if (MAXW) atomicMax(reinterpret_cast<int*>(out.max_w) + vid, __float_as_int(pt_w));
         if (T < kEarlyStopT) {
           done = true;
@@ -247,7 +240,7 @@ __device__ __forceinline__ void render_tile_fwd(const ViewParams& vp, const floa
     uint32_t m = 0;
 #pragma unroll
     for (int w = 0; w < CFG::NW; ++w) m = max(m, s_red[w]);
-    if (SHARED_LAST) atomicMax(last_slot, range.x + m);
+    if (SHARED_LIST) atomicMax(last_slot, range.x + m);
     else *last_slot = range.x + m;
   }
 }

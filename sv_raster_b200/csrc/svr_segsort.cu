@@ -403,13 +403,6 @@ void ensure_segsort_attributes() {
   });
 }
 
-static int sm_count() {
-  int dev = 0, n = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n > 0 ? n : 148;
-}
-
 template <int CHUNK, typename KT>
 static void launch_chunk_and_merge(const SegLists& L, int sms, uint64_t* ka, uint32_t* va, uint64_t* kb,
                                    uint32_t* vb, int rank_bits, cudaStream_t stream) {
