@@ -17,48 +17,112 @@
 
 namespace svr {
 
+// A voxel's rest coefficients (or their gradients) are a row of 3 (M - 1)
+// values, 180 bytes at degree 3: a thread reading or writing its own row alone
+// touches a line of its own with every access.  Each warp moves the rows of its
+// 32 voxels together instead, element after element through shared memory (row
+// strides are odd, so a lane's walk over its row is free of conflicts).  Voxels
+// with consecutive ids then make full-width accesses.  1.93M visible of 2M
+// voxels, degree 3, fp32: the evaluation 117 -> 111 us (its rows came through the
+// L1 cache before), the backward 563 -> 86 us; the rows alone take 56 us at the
+// copy bandwidth.
+constexpr int kShThreads = 128;
+constexpr int kShUnroll = 8;
+
+// Row elements of degree DEG (the coefficients above it are not touched).
+template <int DEG>
+constexpr int sh_row() { return 3 * ((DEG + 1) * (DEG + 1) - 1); }
+template <int DEG>
+constexpr int sh_stride() { return sh_row<DEG>() | 1; }
+
 template <int DEG, typename TS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kShThreads)
 sh_eval_kernel(int n_idx, int P, int M, const int64_t* __restrict__ idx, const float* __restrict__ centers,
                const float* __restrict__ cam_pos, const TS* __restrict__ sh0, const TS* __restrict__ shs,
                float* __restrict__ rgbs) {
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if ((n_idx == 0 && tid >= P) || (n_idx != 0 && tid >= n_idx)) return;
-  const int64_t i = (n_idx != 0) ? idx[tid] : tid;
+  constexpr int ROW = sh_row<DEG>(), STRIDE = sh_stride<DEG>();
+  __shared__ float s_rows[ROW > 0 ? kShThreads * STRIDE : 1];
+  const int n = n_idx != 0 ? n_idx : P;
+  const int tid = blockIdx.x * kShThreads + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const bool on = tid < n;
+  const int64_t i = on ? (n_idx != 0 ? idx[tid] : (int64_t)tid) : 0;
+  float* rows = s_rows + (threadIdx.x & ~31) * STRIDE;
+  if (ROW > 0) {
+    const int n_here = min(32, n - (tid - lane));
+    const int rest = (M - 1) * 3;
+    // Row after row, kShUnroll of them in flight at once; a lane takes elements
+    // lane and lane + 32.
+#pragma unroll 1
+    for (int v0 = 0; v0 < 32; v0 += kShUnroll) {
+      float t[kShUnroll][2];
+#pragma unroll
+      for (int u = 0; u < kShUnroll; ++u) {
+        const TS* row = shs + (size_t)__shfl_sync(0xffffffffu, i, v0 + u) * rest;
+        const bool in = v0 + u < n_here;
+        t[u][0] = in && lane < ROW ? ldf(row, lane) : 0.f;
+        if (ROW > 32) t[u][1] = in && lane + 32 < ROW ? ldf(row, lane + 32) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < kShUnroll; ++u) {
+        float* d = rows + (v0 + u) * STRIDE;
+        if (lane < ROW) d[lane] = t[u][0];
+        if (ROW > 32 && lane + 32 < ROW) d[lane + 32] = t[u][1];
+      }
+    }
+    __syncwarp();
+  }
+  if (!on) return;
   float dx = centers[3 * i + 0] - cam_pos[0];
   float dy = centers[3 * i + 1] - cam_pos[1];
   float dz = centers[3 * i + 2] - cam_pos[2];
   const float rn = rnorm3df(dx, dy, dz);
   dx = dx * rn; dy = dy * rn; dz = dz * rn;
-  const TS* sh = shs + (size_t)i * (M - 1) * 3;
+  const float* sh = rows + lane * STRIDE;
 #pragma unroll
   for (int c = 0; c < 3; ++c) rgbs[3 * i + c] = sh_channel<DEG>(dx, dy, dz, ldf(sh0, 3 * i + c), sh, c);
 }
 
 template <int DEG>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kShThreads)
 sh_eval_bw_kernel(int n_idx, int P, int M, const int64_t* __restrict__ idx, const float* __restrict__ centers,
                   const float* __restrict__ cam_pos, const float* __restrict__ dL_drgbs, float* __restrict__ dL_dsh0,
                   float* __restrict__ dL_dshs) {
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if ((n_idx == 0 && tid >= P) || (n_idx != 0 && tid >= n_idx)) return;
-  const int64_t i = (n_idx != 0) ? idx[tid] : tid;
-  float x = centers[3 * i + 0] - cam_pos[0];
-  float y = centers[3 * i + 1] - cam_pos[1];
-  float z = centers[3 * i + 2] - cam_pos[2];
-  const float rn = rnorm3df(x, y, z);
-  x = x * rn; y = y * rn; z = z * rn;
-  const float g[3] = {dL_drgbs[3 * i + 0], dL_drgbs[3 * i + 1], dL_drgbs[3 * i + 2]};
-  float* d = dL_dshs + (size_t)i * (M - 1) * 3;
-  float basis[15];
-  const int nb = sh_basis_rest<DEG>(x, y, z, basis);
+  constexpr int ROW = sh_row<DEG>(), STRIDE = sh_stride<DEG>();
+  __shared__ float s_rows[ROW > 0 ? kShThreads * STRIDE : 1];
+  const int n = n_idx != 0 ? n_idx : P;
+  const int tid = blockIdx.x * kShThreads + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const bool on = tid < n;
+  const int64_t i = on ? (n_idx != 0 ? idx[tid] : (int64_t)tid) : 0;
+  float* rows = s_rows + (threadIdx.x & ~31) * STRIDE;
+  if (on) {
+    float x = centers[3 * i + 0] - cam_pos[0];
+    float y = centers[3 * i + 1] - cam_pos[1];
+    float z = centers[3 * i + 2] - cam_pos[2];
+    const float rn = rnorm3df(x, y, z);
+    x = x * rn; y = y * rn; z = z * rn;
+    const float g[3] = {dL_drgbs[3 * i + 0], dL_drgbs[3 * i + 1], dL_drgbs[3 * i + 2]};
+    float basis[15];
+    sh_basis_rest<DEG>(x, y, z, basis);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) dL_dsh0[3 * i + c] = kC0 * g[c];
+    for (int c = 0; c < 3; ++c) dL_dsh0[3 * i + c] = kC0 * g[c];
 #pragma unroll
-  for (int k = 0; k < 15; ++k) {
-    if (k >= nb) break;
+    for (int k = 0; k < ROW / 3; ++k)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) d[3 * k + c] = basis[k] * g[c];
+      for (int c = 0; c < 3; ++c) rows[lane * STRIDE + 3 * k + c] = basis[k] * g[c];
+  }
+  if (ROW > 0) {
+    __syncwarp();
+    const int n_here = min(32, n - (tid - lane));
+    const int rest = (M - 1) * 3;
+#pragma unroll 8
+    for (int v = 0; v < n_here; ++v) {
+      float* row = dL_dshs + (size_t)__shfl_sync(0xffffffffu, i, v) * rest;
+      const float* d = rows + v * STRIDE;
+      if (lane < ROW) __stcs(row + lane, d[lane]);
+      if (ROW > 32 && lane + 32 < ROW) __stcs(row + lane + 32, d[lane + 32]);
+    }
   }
 }
 
@@ -66,13 +130,13 @@ void launch_sh_eval(int deg, int n_idx, int P, int M, const int64_t* idx, const 
                     const void* sh0, const void* shs, bool bf16, float* rgbs, cudaStream_t stream) {
   const int n = n_idx != 0 ? n_idx : P;
   if (n <= 0) return;
-  const int g = (n + 255) / 256;
+  const int g = (n + kShThreads - 1) / kShThreads;
 #define SVR_SH_L(D)                                                                                            \
   if (bf16)                                                                                                    \
-    sh_eval_kernel<D, __nv_bfloat16><<<g, 256, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos,                \
+    sh_eval_kernel<D, __nv_bfloat16><<<g, kShThreads, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos,                \
                                                             (const __nv_bfloat16*)sh0, (const __nv_bfloat16*)shs, rgbs); \
   else                                                                                                         \
-    sh_eval_kernel<D, float><<<g, 256, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos, (const float*)sh0,     \
+    sh_eval_kernel<D, float><<<g, kShThreads, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos, (const float*)sh0,     \
                                                     (const float*)shs, rgbs);
   switch (deg) {
     case 0: SVR_SH_L(0) break;
@@ -88,12 +152,12 @@ void launch_sh_eval_bw(int deg, int n_idx, int P, int M, const int64_t* idx, con
                        cudaStream_t stream) {
   const int n = n_idx != 0 ? n_idx : P;
   if (n <= 0) return;
-  const int g = (n + 255) / 256;
+  const int g = (n + kShThreads - 1) / kShThreads;
   switch (deg) {
-    case 0: sh_eval_bw_kernel<0><<<g, 256, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos, dL_drgbs, dL_dsh0, dL_dshs); break;
-    case 1: sh_eval_bw_kernel<1><<<g, 256, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos, dL_drgbs, dL_dsh0, dL_dshs); break;
-    case 2: sh_eval_bw_kernel<2><<<g, 256, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos, dL_drgbs, dL_dsh0, dL_dshs); break;
-    default: sh_eval_bw_kernel<3><<<g, 256, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos, dL_drgbs, dL_dsh0, dL_dshs); break;
+    case 0: sh_eval_bw_kernel<0><<<g, kShThreads, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos, dL_drgbs, dL_dsh0, dL_dshs); break;
+    case 1: sh_eval_bw_kernel<1><<<g, kShThreads, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos, dL_drgbs, dL_dsh0, dL_dshs); break;
+    case 2: sh_eval_bw_kernel<2><<<g, kShThreads, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos, dL_drgbs, dL_dsh0, dL_dshs); break;
+    default: sh_eval_bw_kernel<3><<<g, kShThreads, 0, stream>>>(n_idx, P, M, idx, centers, cam_pos, dL_drgbs, dL_dsh0, dL_dshs); break;
   }
 }
 
@@ -104,59 +168,108 @@ __device__ __forceinline__ float adam_lerp(float v0, float v1, float t) {
   return fmaf(t, v1, fmaf(-t, v0, v0));  // (1-t)*v0 + t*v1, adam_step.cu:21-25
 }
 
-template <bool SPARSE>
-__global__ void __launch_bounds__(256)
-adam_unbiased_kernel(int64_t numel, float* __restrict__ param, const float* __restrict__ grad,
-                     float* __restrict__ exp_avg, float* __restrict__ exp_avg_sq, float step_size, float beta1,
-                     float beta2, float rsqrt_bc2, float eps) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// One element's update (adam_step.cu:28-102): `scale` is the step size
+// (unbiased) or the learning rate (biased).
+template <bool BIASED>
+__device__ __forceinline__ void adam_element(float g, float& p, float& m, float& v, float scale, float beta1,
+                                             float beta2, float rsqrt_bc2, float eps) {
+  m = adam_lerp(g, m, beta1);
+  v = adam_lerp(g * g, v, beta2);
+  const float denom = BIASED ? sqrtf(v) + eps : fmaf(sqrtf(v), rsqrt_bc2, eps);
+  p -= scale * (m / denom);
+}
+
+// Four elements per access where the four arrays are 16-byte aligned (VEC), and
+// kAdamUnroll accesses of a thread in flight at once; with SPARSE, four zero
+// gradients read nothing else.  Streams 4 B per element and 24 B more per touched
+// one, each once, so past the cache.  118M elements, 40 % of the voxels touched:
+// 706 us with one element per thread, 354 here (4.5 TB/s; 367 without the
+// streaming hints, 404 and 468 with 1 and 4 accesses in flight).
+constexpr int kAdamThreads = 256;
+constexpr int kAdamUnroll = 2;
+
+template <bool BIASED, bool SPARSE>
+__global__ void __launch_bounds__(kAdamThreads)
+adam_vec_kernel(int64_t n4, float4* __restrict__ param, const float4* __restrict__ grad, float4* __restrict__ exp_avg,
+                float4* __restrict__ exp_avg_sq, float scale, float beta1, float beta2, float rsqrt_bc2, float eps) {
+  const int64_t base = (int64_t)blockIdx.x * (kAdamThreads * kAdamUnroll) + threadIdx.x;
+  float4 g[kAdamUnroll], p[kAdamUnroll], m[kAdamUnroll], v[kAdamUnroll];
+  bool on[kAdamUnroll];
+#pragma unroll
+  for (int u = 0; u < kAdamUnroll; ++u) {
+    const int64_t i = base + u * kAdamThreads;
+    on[u] = i < n4;
+    if (on[u]) g[u] = __ldcs(grad + i);
+  }
+#pragma unroll
+  for (int u = 0; u < kAdamUnroll; ++u) {
+    const int64_t i = base + u * kAdamThreads;
+    if (SPARSE) on[u] = on[u] && !(g[u].x == 0.f && g[u].y == 0.f && g[u].z == 0.f && g[u].w == 0.f);
+    if (on[u]) {
+      p[u] = __ldcs(param + i);
+      m[u] = __ldcs(exp_avg + i);
+      v[u] = __ldcs(exp_avg_sq + i);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kAdamUnroll; ++u) {
+    if (!on[u]) continue;
+    const int64_t i = base + u * kAdamThreads;
+    const auto step = [&](float ge, float& pe, float& me, float& ve) {
+      if (!SPARSE || ge != 0.f) adam_element<BIASED>(ge, pe, me, ve, scale, beta1, beta2, rsqrt_bc2, eps);
+    };
+    step(g[u].x, p[u].x, m[u].x, v[u].x);
+    step(g[u].y, p[u].y, m[u].y, v[u].y);
+    step(g[u].z, p[u].z, m[u].z, v[u].z);
+    step(g[u].w, p[u].w, m[u].w, v[u].w);
+    __stcs(param + i, p[u]);
+    __stcs(exp_avg + i, m[u]);
+    __stcs(exp_avg_sq + i, v[u]);
+  }
+}
+
+// The elements past the last group of four, and arrays that are not 16-byte
+// aligned.
+template <bool BIASED, bool SPARSE>
+__global__ void __launch_bounds__(kAdamThreads)
+adam_scalar_kernel(int64_t first, int64_t numel, float* __restrict__ param, const float* __restrict__ grad,
+                   float* __restrict__ exp_avg, float* __restrict__ exp_avg_sq, float scale, float beta1, float beta2,
+                   float rsqrt_bc2, float eps) {
+  const int64_t i = first + (int64_t)blockIdx.x * kAdamThreads + threadIdx.x;
   if (i >= numel) return;
   const float g = grad[i];
   if (SPARSE && g == 0.0f) return;
-  float m = exp_avg[i];
-  float v = exp_avg_sq[i];
-  m = adam_lerp(g, m, beta1);
-  v = adam_lerp(g * g, v, beta2);
-  const float denom = fmaf(sqrtf(v), rsqrt_bc2, eps);
-  const float step = step_size * (m / denom);
-  param[i] -= step;
+  float p = param[i], m = exp_avg[i], v = exp_avg_sq[i];
+  adam_element<BIASED>(g, p, m, v, scale, beta1, beta2, rsqrt_bc2, eps);
+  param[i] = p;
   exp_avg[i] = m;
   exp_avg_sq[i] = v;
 }
 
-template <bool SPARSE>
-__global__ void __launch_bounds__(256)
-adam_biased_kernel(int64_t numel, float* __restrict__ param, const float* __restrict__ grad,
-                   float* __restrict__ exp_avg, float* __restrict__ exp_avg_sq, float lr, float beta1, float beta2,
-                   float eps) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= numel) return;
-  const float g = grad[i];
-  if (SPARSE && g == 0.0f) return;
-  float m = exp_avg[i];
-  float v = exp_avg_sq[i];
-  m = adam_lerp(g, m, beta1);
-  v = adam_lerp(g * g, v, beta2);
-  const float denom = sqrtf(v) + eps;
-  const float step = lr * (m / denom);
-  param[i] -= step;
-  exp_avg[i] = m;
-  exp_avg_sq[i] = v;
+template <bool BIASED, bool SPARSE>
+static void adam_run(int64_t numel, float* param, const float* grad, float* m, float* v, float scale, float beta1,
+                     float beta2, float rsqrt_bc2, float eps, cudaStream_t stream) {
+  const auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  const bool vec = aligned(param) && aligned(grad) && aligned(m) && aligned(v);
+  const int64_t n4 = vec ? numel / 4 : 0;
+  if (n4 > 0) {
+    constexpr int64_t per = kAdamThreads * kAdamUnroll;
+    adam_vec_kernel<BIASED, SPARSE><<<(unsigned)((n4 + per - 1) / per), kAdamThreads, 0, stream>>>(
+        n4, reinterpret_cast<float4*>(param), reinterpret_cast<const float4*>(grad), reinterpret_cast<float4*>(m),
+        reinterpret_cast<float4*>(v), scale, beta1, beta2, rsqrt_bc2, eps);
+  }
+  if (4 * n4 < numel)
+    adam_scalar_kernel<BIASED, SPARSE>
+        <<<(unsigned)((numel - 4 * n4 + kAdamThreads - 1) / kAdamThreads), kAdamThreads, 0, stream>>>(
+            4 * n4, numel, param, grad, m, v, scale, beta1, beta2, rsqrt_bc2, eps);
 }
 
 void launch_adam(bool biased, bool sparse, int64_t numel, float* param, const float* grad, float* m, float* v,
                  float step_or_lr, float beta1, float beta2, float rsqrt_bc2, float eps, cudaStream_t stream) {
   if (numel <= 0) return;
-  const unsigned g = (unsigned)((numel + 255) / 256);
-  if (biased) {
-    if (sparse) adam_biased_kernel<true><<<g, 256, 0, stream>>>(numel, param, grad, m, v, step_or_lr, beta1, beta2, eps);
-    else adam_biased_kernel<false><<<g, 256, 0, stream>>>(numel, param, grad, m, v, step_or_lr, beta1, beta2, eps);
-  } else {
-    if (sparse)
-      adam_unbiased_kernel<true><<<g, 256, 0, stream>>>(numel, param, grad, m, v, step_or_lr, beta1, beta2, rsqrt_bc2, eps);
-    else
-      adam_unbiased_kernel<false><<<g, 256, 0, stream>>>(numel, param, grad, m, v, step_or_lr, beta1, beta2, rsqrt_bc2, eps);
-  }
+  const auto run = biased ? (sparse ? adam_run<true, true> : adam_run<true, false>)
+                          : (sparse ? adam_run<false, true> : adam_run<false, false>);
+  run(numel, param, grad, m, v, step_or_lr, beta1, beta2, rsqrt_bc2, eps, stream);
 }
 
 // Fused multi-group Adam: one launch walks every group's elements with
@@ -189,6 +302,7 @@ adam_fused_kernel(const __grid_constant__ AdamGroupTable t) {
     float g4[4], m4[4], v4[4], p4[4];
     if (full) {
       *reinterpret_cast<float4*>(g4) = reinterpret_cast<const float4*>(G.grad)[q];
+      if (t.sparse && g4[0] == 0.f && g4[1] == 0.f && g4[2] == 0.f && g4[3] == 0.f) continue;
       *reinterpret_cast<float4*>(m4) = reinterpret_cast<const float4*>(G.exp_avg)[q];
       *reinterpret_cast<float4*>(v4) = reinterpret_cast<const float4*>(G.exp_avg_sq)[q];
       if (G.param_bf16) {
@@ -267,7 +381,10 @@ void launch_adam_fused(const AdamGroupTable& t, int num_sms, cudaStream_t stream
 // and write its 8 outputs as one contiguous run, so key reads and output
 // stores are coalesced across the warp; only the grid-point reads (and the
 // backward's adds) are scattered.  Each thread carries U slots, 256 apart,
-// through every load stage together so U scattered reads are in flight.
+// through every load stage together so U scattered reads are in flight.  What is
+// streamed once passes by the L2 cache, which is left to the grid points, and
+// zero gradients (voxels a view does not see) add nothing: 2M voxels, 10M grid
+// points, 40 % seen: gather 55 -> 53 us, its backward 58 -> 41 us.
 constexpr int kGatherThreads = 256;
 
 template <int DIM, int U>
@@ -283,7 +400,7 @@ gather_kernel(int64_t n_slots, const int64_t* __restrict__ vox_key, const int64_
     slot[j] = t < n_slots ? 8 * care_idx[t >> 3] + (t & 7) : -1;
   }
 #pragma unroll
-  for (int j = 0; j < U; ++j) k[j] = slot[j] >= 0 ? vox_key[slot[j]] : 0;
+  for (int j = 0; j < U; ++j) k[j] = slot[j] >= 0 ? __ldcs(vox_key + slot[j]) : 0;
 #pragma unroll
   for (int j = 0; j < U; ++j)
 #pragma unroll
@@ -292,7 +409,7 @@ gather_kernel(int64_t n_slots, const int64_t* __restrict__ vox_key, const int64_
   for (int j = 0; j < U; ++j)
     if (slot[j] >= 0)
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) out[slot[j] * DIM + d] = v[j][d];
+      for (int d = 0; d < DIM; ++d) __stcs(out + slot[j] * DIM + d, v[j][d]);
 }
 
 template <int DIM, int U>
@@ -309,15 +426,16 @@ gather_bw_kernel(int64_t n_slots, const int64_t* __restrict__ vox_key, const int
   }
 #pragma unroll
   for (int j = 0; j < U; ++j) {
-    k[j] = slot[j] >= 0 ? vox_key[slot[j]] : 0;
+    k[j] = slot[j] >= 0 ? __ldcs(vox_key + slot[j]) : 0;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) g[j][d] = slot[j] >= 0 ? dL_dvox[slot[j] * DIM + d] : 0.f;
+    for (int d = 0; d < DIM; ++d) g[j][d] = slot[j] >= 0 ? __ldcs(dL_dvox + slot[j] * DIM + d) : 0.f;
   }
 #pragma unroll
   for (int j = 0; j < U; ++j)
     if (slot[j] >= 0)
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) atomicAdd(dL_dgrid + k[j] * DIM + d, g[j][d]);
+      for (int d = 0; d < DIM; ++d)
+        if (g[j][d] != 0.f) atomicAdd(dL_dgrid + k[j] * DIM + d, g[j][d]);  // unseen voxels bring zeros
 }
 
 template <int DIM, int U, class KERNEL>

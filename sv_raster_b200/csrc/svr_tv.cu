@@ -63,7 +63,7 @@ tv_grad_kernel(int64_t n_slots, int C, const float* __restrict__ grid, const int
   for (int j = 0; j < kTvSlots; ++j) {
     const int64_t t = base + j * kTvThreads, nc = t >> 3;
     const bool on = t < n_slots && (!active || active[nc]);  // uniform over the 8 lanes of a group
-    at[j] = on ? vox_key[8 * (nc / C) + (t & 7)] * C + nc % C : -1;
+    at[j] = on ? __ldcs(vox_key + 8 * (nc / C) + (t & 7)) * C + nc % C : -1;
     w[j] = weight;
     if (SCALE && on) w[j] *= 0.01f * vox_size_inv[nc / C];
   }
