@@ -7,8 +7,8 @@
 // the results are those of the plain path:
 //   - projection is project_voxel (preprocess.cu:24-132 arithmetic), fused
 //     with the SH colour of each visible (voxel, view) (sh_compute.cu:54-106);
-//   - instances of all views share one flat array, view-major, keyed
-//     [tile | rank position]: the position of the instance's (voxel,
+//   - instances of all views share one flat array, tile after tile, sorted
+//     inside a tile by rank position: the position of the instance's (voxel,
 //     quadrant) pair in the ascending order of all 8P pairs' Morton ranks
 //     (ties by voxel, then quadrant: the reference's generation order).  The
 //     positions are view-independent, built once per plan by one radix sort,
@@ -18,6 +18,7 @@
 //     bits are the quadrant repeated, so (rank >> 3*(16-L)) << 3 | quadrant
 //     orders pairs exactly as the full rank does;
 //   - compositing / backward are the same per-tile device functions.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
@@ -54,17 +55,45 @@ struct GroupTable {
 // ---------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------
-// One thread per voxel, looping over the views: the voxel's centre, size and
-// SH coefficients are read once (the coefficients on its first visible view)
-// and kept in registers, so each view costs the projection arithmetic and
-// the per-(view, voxel) writes only.
+// Tiles of a pixel bbox in one view, numbered row by row (none when not on).
+constexpr uint32_t kOwnTiles = 4;  // pairs of at most this many tiles: handled by their own thread
+struct TileRect {
+  uint32_t first, w, n, pitch;
+  __device__ __forceinline__ TileRect() {}
+  __device__ __forceinline__ TileRect(uint2 bbox, const ViewParams& vp, bool on) : first(0), w(1), n(0), pitch(0) {
+    if (!on) return;
+    int x0, y0, x1, y1;
+    bbox_tile_rect(bbox, vp.grid_x, vp.grid_y, vp.tile_shift, x0, y0, x1, y1);
+    pitch = (uint32_t)vp.grid_x;
+    first = (uint32_t)y0 * pitch + (uint32_t)x0;
+    w = (uint32_t)(x1 - x0 + 1);
+    n = w * (uint32_t)(y1 - y0 + 1);
+  }
+  __device__ __forceinline__ uint32_t tile(uint32_t k) const { return first + k / w * pitch + k % w; }
+  __device__ __forceinline__ TileRect from(int lane) const {
+    TileRect r;
+    r.first = __shfl_sync(0xffffffffu, first, lane);
+    r.w = __shfl_sync(0xffffffffu, w, lane);
+    r.n = __shfl_sync(0xffffffffu, n, lane);
+    r.pitch = __shfl_sync(0xffffffffu, pitch, lane);
+    return r;
+  }
+};
+
+// One thread per voxel, looping over the views: the voxel's centre and size are
+// read once and kept in registers, so each view costs the projection arithmetic
+// and the per-(view, voxel) writes only.
+// With `counts`, every visible pair also adds its instances to its tiles' counts
+// (a warp takes the pairs of many tiles together, one tile per lane): 1.78 -> 2.22
+// ms for 8M voxels and eight views, where counting in a pass of its own, which
+// re-read 20 bytes per pair, took 0.88.
 template <int DEG, typename TS>
 __global__ void __launch_bounds__(128)
 project_sh_kernel(const __grid_constant__ ViewTable views, int P, const float* __restrict__ centers,
                   const float* __restrict__ lengths, const TS* __restrict__ sh0, const TS* __restrict__ shs, int M,
                   const int64_t* __restrict__ octpaths, int level_low_bits, int tight, uint32_t* __restrict__ ndup,
                   uint2* __restrict__ bboxes, uint32_t* __restrict__ quads, float* __restrict__ rgbs,
-                  uint32_t* __restrict__ err, unsigned long long* __restrict__ pixels) {
+                  uint32_t* __restrict__ err, unsigned long long* __restrict__ pixels, uint32_t* __restrict__ counts) {
   __shared__ float s_m[kMaxViews][24];           // w2c (12) and c2w (12) of every view
   __shared__ unsigned long long s_pixels;
   if (threadIdx.x == 0) s_pixels = 0ull;
@@ -74,46 +103,126 @@ project_sh_kernel(const __grid_constant__ ViewTable views, int P, const float* _
   }
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool in = i < P;
+  const size_t iv = in ? i : 0;
   uint32_t px = 0u;  // bbox pixels over the views (each at most 2^20 here: a warp's sum fits 32 bits)
-  if (i < P) {
-    // voxels deeper than the plan's max level would break the compressed ranks
-    if (level_low_bits > 0 && ((uint64_t)octpaths[i] & ((1ull << level_low_bits) - 1ull)) != 0ull)
-      atomicOr(err, SVR_DEVERR_LEVEL);
-    const float cx = centers[3 * (size_t)i], cy = centers[3 * (size_t)i + 1], cz = centers[3 * (size_t)i + 2];
-    const float len = lengths[i];
-    // The rest coefficients are read per visible view through the cache
-    // (holding 45 of them in registers across the views cost the kernel half
-    // its occupancy).
-    const TS* sh = shs + (size_t)i * (M - 1) * 3;
-    float c0[3];
-    bool loaded = false;
-    for (int v = 0; v < views.n; ++v) {
-      const size_t o = (size_t)v * P + i;
-      const float* m = s_m[v];
-      Projection pr = project_voxel(views.v[v], m, m + 12, cx, cy, cz, len);
-      if (tight) tighten_bbox(views.v[v], pr);
+  // voxels deeper than the plan's max level would break the compressed ranks
+  if (level_low_bits > 0 && in && ((uint64_t)octpaths[iv] & ((1ull << level_low_bits) - 1ull)) != 0ull)
+    atomicOr(err, SVR_DEVERR_LEVEL);
+  const float cx = centers[3 * iv], cy = centers[3 * iv + 1], cz = centers[3 * iv + 2];
+  const float len = lengths[iv];
+  // The rest coefficients are read per visible view through the cache: holding
+  // 45 of them in registers across the views cost the kernel half its occupancy,
+  // and staging the rows in shared memory was slower with one view (123 -> 218
+  // us, 2M voxels) and no faster with eight.
+  const TS* sh = shs + iv * (M - 1) * 3;
+  float c0[3];
+  bool loaded = false;
+  for (int v = 0; v < views.n; ++v) {
+    const size_t o = (size_t)v * P + iv;
+    const float* m = s_m[v];
+    Projection pr = project_voxel(views.v[v], m, m + 12, cx, cy, cz, len);
+    if (tight) tighten_bbox(views.v[v], pr);
+    if (in) {
       ndup[o] = pr.n;
       bboxes[o] = pr.bbox;
       quads[o] = pr.quads;
-      if (pr.n == 0) continue;
-      if (!loaded) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) c0[c] = ldf(sh0, 3 * (size_t)i + c);
-        loaded = true;
-      }
-      // View-dependent colour of this visible voxel (sh_compute.cu:54-106).
-      float dx = cx - m[12 + 3], dy = cy - m[12 + 7], dz = cz - m[12 + 11];
-      const float rn = rnorm3df(dx, dy, dz);
-      dx = dx * rn; dy = dy * rn; dz = dz * rn;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) rgbs[3 * o + c] = sh_channel<DEG>(dx, dy, dz, c0[c], sh, c);
-      px += min((bb_xmax(pr.bbox) - bb_xmin(pr.bbox) + 1u) * (bb_ymax(pr.bbox) - bb_ymin(pr.bbox) + 1u), 1u << 20);
     }
+    const bool visible = in && pr.n != 0;
+    if (counts) {
+      const TileRect rect(pr.bbox, views.v[v], visible);
+      const uint32_t per_tile = (uint32_t)__popc(pr.quads);
+      uint32_t* c = counts + views.v[v].tile_base;
+      if (rect.n <= kOwnTiles) {
+        uint32_t t = rect.first, left = rect.w;
+        for (uint32_t k = 0; k < rect.n; ++k) {
+          atomicAdd(c + t, per_tile);
+          ++t;
+          if (--left == 0) {
+            left = rect.w;
+            t += rect.pitch - rect.w;
+          }
+        }
+      }
+      for (uint32_t big = __ballot_sync(0xffffffffu, rect.n > kOwnTiles); big; big &= big - 1) {
+        const int src = __ffs(big) - 1;
+        const TileRect r = rect.from(src);
+        const uint32_t q = __shfl_sync(0xffffffffu, per_tile, src);
+        for (uint32_t k = threadIdx.x & 31; k < r.n; k += 32) atomicAdd(c + r.tile(k), q);
+      }
+    }
+    if (!visible) continue;
+    if (!loaded) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) c0[c] = ldf(sh0, 3 * iv + c);
+      loaded = true;
+    }
+    // View-dependent colour of this visible voxel (sh_compute.cu:54-106).
+    float dx = cx - m[12 + 3], dy = cy - m[12 + 7], dz = cz - m[12 + 11];
+    const float rn = rnorm3df(dx, dy, dz);
+    dx = dx * rn; dy = dy * rn; dz = dz * rn;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) rgbs[3 * o + c] = sh_channel<DEG>(dx, dy, dz, c0[c], sh, c);
+    px += min((bb_xmax(pr.bbox) - bb_xmin(pr.bbox) + 1u) * (bb_ymax(pr.bbox) - bb_ymin(pr.bbox) + 1u), 1u << 20);
   }
+  __syncwarp();
   px = __reduce_add_sync(0xffffffffu, px);
   if ((threadIdx.x & 31) == 0 && px) atomicAdd(&s_pixels, (unsigned long long)px);
   __syncthreads();
   if (threadIdx.x == 0 && s_pixels) atomicAdd(pixels + blockIdx.x % kCoverageSlots, s_pixels);
+}
+
+// Counting-sort scatter: the rank position of every instance to the next free
+// place of its tile's range (cursor[global tile], starting at the range's
+// start).  Places inside a tile follow the atomics' order; the tile sort orders
+// them.  Places past the capacity are left out (the range scan flagged it).
+// Pairs of few tiles keep their atomics in flight together; a warp takes the
+// others tile by tile, one per lane.  Bound by the returning atomics: 60M
+// instances in 1.16 ms, where a lane per instance, decoded from a scan of all
+// pairs, with keys and values to store took 1.46 and the scan 0.35.
+__global__ void __launch_bounds__(256)
+scatter_positions_kernel(const __grid_constant__ ViewTable views, int P, const uint32_t* __restrict__ rank_pos,
+                         const uint2* __restrict__ bboxes, const uint32_t* __restrict__ quads,
+                         uint32_t* __restrict__ cursor, uint32_t* __restrict__ keys, uint32_t cap) {
+  const ViewParams& vp = views.v[blockIdx.y];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const size_t o = (size_t)blockIdx.y * P + i;
+  const uint32_t qb = i < P ? quads[o] : 0u;
+  if (__ballot_sync(0xffffffffu, qb != 0u) == 0u) return;
+  const TileRect rect(qb ? bboxes[o] : make_uint2(0u, 0u), vp, qb != 0u);
+  uint32_t* c = cursor + vp.tile_base;
+  if (rect.n <= kOwnTiles) {
+    for (uint32_t qs = qb; qs; qs &= qs - 1) {
+      const uint32_t pos = rank_pos[8 * (size_t)i + (__ffs(qs) - 1)];
+      uint32_t at[kOwnTiles];
+      uint32_t t = rect.first, left = rect.w;
+#pragma unroll
+      for (uint32_t k = 0; k < kOwnTiles; ++k) {
+        if (k < rect.n) at[k] = atomicAdd(c + t, 1u);
+        ++t;
+        if (--left == 0) {
+          left = rect.w;
+          t += rect.pitch - rect.w;
+        }
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kOwnTiles; ++k)
+        if (k < rect.n && at[k] < cap) keys[at[k]] = pos;
+    }
+  }
+  for (uint32_t big = __ballot_sync(0xffffffffu, rect.n > kOwnTiles); big; big &= big - 1) {
+    const int src = __ffs(big) - 1;
+    const TileRect r = rect.from(src);
+    const size_t vox = (size_t)(i - lane + src);
+    for (uint32_t qs = __shfl_sync(0xffffffffu, qb, src); qs; qs &= qs - 1) {
+      const uint32_t pos = rank_pos[8 * vox + (__ffs(qs) - 1)];
+      for (uint32_t k = lane; k < r.n; k += 32) {
+        const uint32_t at = atomicAdd(c + r.tile(k), 1u);
+        if (at < cap) keys[at] = pos;
+      }
+    }
+  }
 }
 
 // Instance segment [start, start + count) of each sort group, clamped to the
@@ -144,32 +253,18 @@ __device__ __forceinline__ int nth_set_bit(uint32_t m, int k) {
   return pos;
 }
 
-// Duplication with the stores of a warp coalesced.  The instances of the
-// warp's 32 consecutive (view, voxel) pairs form one contiguous run of the
-// scan; the warp walks that run 32 instances at a time, each lane decoding
-// its instance (owning voxel, then quadrant / tile row / tile column in the
-// plain path's generation order: quadrants ascending, tiles row-major,
-// forward.cu:540-562).  MODE selects what happens to the decoded instance:
-//   kDupWrite   key and value at its own slot (generation order, for the
-//               radix sort over the tile bits);
-//   kDupCount   +1 on its tile's instance count (counts[global tile]);
-//   kDupScatter key and value at the next free position of its tile's range
-//               (ranges[t].y is the tile's cursor, starting at ranges[t].x).
-// Count and scatter aggregate the lanes of a warp that hit the same tile
-// (match.any) into one atomic.  Both skip exactly the instances whose
-// generation slot is beyond the capacity, so every tile's cursor ends at the
-// end of its range.  Positions inside a tile follow the atomics' order; the
-// per-tile segment sort that follows orders them by their unique rank
-// positions, so the final lists do not depend on it.
-constexpr int kDupWrite = 0, kDupCount = 1, kDupScatter = 2;
-
-template <int MODE>
+// Duplication for the radix grouping by tile, with the stores of a warp
+// coalesced.  The instances of the warp's 32 consecutive (view, voxel) pairs form
+// one contiguous run of the scan; the warp walks that run 32 instances at a time,
+// each lane decoding its instance (owning voxel, then quadrant / tile row / tile
+// column in the plain path's generation order: quadrants ascending, tiles
+// row-major, forward.cu:540-562) and writing its key and value at its slot.
 __global__ void __launch_bounds__(256)
 duplicate_batch_kernel(const __grid_constant__ ViewTable views, int P, const uint32_t* __restrict__ rank_pos,
                        const uint2* __restrict__ bboxes, const uint32_t* __restrict__ quads,
                        const uint32_t* __restrict__ ndup, const uint32_t* __restrict__ scan,
                        uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t cap,
-                       uint32_t* __restrict__ err, uint32_t* __restrict__ counts, uint2* __restrict__ ranges) {
+                       uint32_t* __restrict__ err) {
   const int view = blockIdx.y;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -224,41 +319,11 @@ duplicate_batch_kernel(const __grid_constant__ ViewTable views, int P, const uin
       vid = (uint32_t)(blockIdx.x * blockDim.x + (threadIdx.x & ~31) + sl);
       local = ty * (uint32_t)vp.grid_x + tx;
     }
-    if (MODE == kDupWrite) {
-      if (active) {
-        keys[slot] = ((uint64_t)(vp.sort_tile_off + local) << kPosShift) | rank_pos[8 * (size_t)vid + q];
-        vals[slot] = make_sort_val(vid, q);
-      }
-    } else {
-      // global tile of the instance; inactive lanes share a value no tile has
-      const uint32_t gtile = active ? vp.tile_base + local : 0xffffffffu;
-      const uint32_t peers = __match_any_sync(0xffffffffu, gtile);
-      const int leader = __ffs(peers) - 1;
-      if (MODE == kDupCount) {
-        if (active && lane == leader) atomicAdd(counts + gtile, (uint32_t)__popc(peers));
-      } else {
-        uint32_t base = 0;
-        if (active && lane == leader) base = atomicAdd(&ranges[gtile].y, (uint32_t)__popc(peers));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (active) {
-          const uint32_t pos = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-          keys[pos] = ((uint64_t)(vp.sort_tile_off + local) << kPosShift) | rank_pos[8 * (size_t)vid + q];
-          vals[pos] = make_sort_val(vid, q);
-        }
-      }
+    if (active) {
+      keys[slot] = ((uint64_t)(vp.sort_tile_off + local) << kPosShift) | rank_pos[8 * (size_t)vid + q];
+      vals[slot] = make_sort_val(vid, q);
     }
   }
-}
-
-// Binned ranges: from each tile's instance count and its inclusive scan,
-// ranges[t] = (start, start); the scatter pass advances .y to the end.  Empty
-// tiles get (0, 0), as the radix path leaves them.
-__global__ void bin_ranges_kernel(uint32_t n_tiles, const uint32_t* __restrict__ counts,
-                                  const uint32_t* __restrict__ incl, uint2* __restrict__ ranges) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_tiles) return;
-  const uint32_t n = counts[t], start = n ? incl[t] - n : 0u;
-  ranges[t] = make_uint2(start, start);
 }
 
 // Rank-position table, step 1: the (compressed) Morton rank of every
@@ -278,11 +343,15 @@ __global__ void rank_pos_keys_kernel(int P, const int64_t* __restrict__ octpaths
   vals[i] = (uint32_t)i;
 }
 
-// Step 2: after a stable sort of the keys, position k holds pair vals[k].
+// Step 2: after a stable sort of the keys, position k holds pair vals[k]; back
+// from a position to its instance value (quadrant | voxel).
 __global__ void rank_pos_scatter_kernel(size_t n, const uint32_t* __restrict__ sorted_pairs,
-                                        uint32_t* __restrict__ rank_pos) {
+                                        uint32_t* __restrict__ rank_pos, uint32_t* __restrict__ val_of_pos) {
   const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) rank_pos[sorted_pairs[k]] = (uint32_t)k;
+  if (k >= n) return;
+  const uint32_t pair = sorted_pairs[k];
+  rank_pos[pair] = (uint32_t)k;
+  val_of_pos[k] = make_sort_val(pair >> 3, pair & 7u);
 }
 
 // dL/dSH of every voxel summed over views: sum_v basis(dir_v) * dL/drgb_v
@@ -401,7 +470,7 @@ struct svr_batch_plan {
   // workspace layout (byte offsets)
   size_t o_header, o_ndup, o_scan, o_bbox, o_quad, o_scan_tmp, o_rgbs, o_drgbs;
   size_t o_ka, o_kb, o_va, o_vb, o_sort_tmp, o_ranges, o_tile_last, o_ncontrib;
-  size_t o_okey, o_oval, o_order_fwd, o_order_bwd, o_order_tmp, o_pos;
+  size_t o_okey, o_oval, o_order_fwd, o_order_bwd, o_order_tmp, o_pos, o_valpos;
   size_t bytes;
 };
 
@@ -428,7 +497,17 @@ struct BatchPtrs {
   uint32_t* order_bwd;  // [T]
   void* order_tmp;
   uint32_t* rank_pos;   // [8P] position of (voxel, quadrant) in rank order
+  uint32_t* val_of_pos; // [8P] instance value of a position
+  uint32_t* counts;     // [T] instances per tile, then the scatter's cursors (after the header)
 };
+
+// Header words: [0] instance count, [1] error word, [2] forward work counter,
+// [3] backward work counter, [4] tile count read by the order sort, [5] pair
+// count read by the rank-position sort, [6] listed runs of long tiles
+// (counting sort), [16..] group segments, then the 64-bit pixel counts of
+// CoverageCount.  The tile counts follow.
+constexpr int kCoverageWord = 16 + 2 * kMaxViews;
+constexpr int kHeaderWords = kCoverageWord + 2 * kCoverageSlots;
 
 BatchPtrs ptrs(const svr_batch_plan* p, void* ws) {
   char* b = static_cast<char*>(ws);
@@ -455,25 +534,26 @@ BatchPtrs ptrs(const svr_batch_plan* p, void* ws) {
   q.order_bwd = reinterpret_cast<uint32_t*>(b + p->o_order_bwd);
   q.order_tmp = b + p->o_order_tmp;
   q.rank_pos = reinterpret_cast<uint32_t*>(b + p->o_pos);
+  q.val_of_pos = reinterpret_cast<uint32_t*>(b + p->o_valpos);
+  q.counts = q.header + kHeaderWords;
   return q;
 }
 
-// Header words: [0] instance count, [1] error word, [2] forward work counter,
-// [3] backward work counter, [4] tile count read by the order sort, [5] pair
-// count read by the rank-position sort, [6] binned instance count (counting
-// sort by tile), [16..] group segments, then the 64-bit pixel counts of
-// CoverageCount.
-constexpr int kCoverageWord = 16 + 2 * kMaxViews;
-constexpr int kHeaderWords = kCoverageWord + 2 * kCoverageSlots;
 unsigned long long* coverage_words(const BatchPtrs& q) {
   return reinterpret_cast<unsigned long long*>(q.header + kCoverageWord);
 }
 
-// Longest-first work order of all tiles into `order` (see launch_tile_order).
+// Largest-first work order of all tiles into `order`, and the work counter back
+// to zero.
 void build_tile_order(const svr_batch_plan* p, const BatchPtrs& q, const uint32_t* tile_last, uint32_t* order,
-                      cudaStream_t stream) {
-  launch_tile_order(q.ranges, tile_last, (uint32_t)p->total_tiles, q.okey, q.oval, order, q.header + 4, q.order_tmp,
-                    stream);
+                      uint32_t* counter, cudaStream_t stream) {
+  const uint32_t T = (uint32_t)p->total_tiles;
+  if (small_tile_order_fits(T)) {
+    launch_small_tile_order(q.ranges, tile_last, T, order, counter, stream);
+    return;
+  }
+  cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream);
+  launch_tile_order(q.ranges, tile_last, T, q.okey, q.oval, order, q.header + 4, q.order_tmp, stream);
 }
 
 inline int check_last() { return cudaGetLastError() == cudaSuccess ? SVR_OK : SVR_ERR_CUDA; }
@@ -577,12 +657,12 @@ int svr_batch_plan_create(int n_views, const svr_camera* cams, int64_t P, int64_
     off += bytes;
     return r;
   };
-  p->o_header = take(kHeaderWords * sizeof(uint32_t));
+  p->o_header = take((kHeaderWords + (size_t)tiles) * sizeof(uint32_t));
   p->o_ndup = take(VP * 4);
   p->o_scan = take(VP * 4);
   p->o_bbox = take(VP * 8);
   p->o_quad = take(VP * 4);
-  p->o_scan_tmp = take(scan_temp_bytes(std::max(VP, (size_t)tiles)));  // instance scan, then the tile-count scan
+  p->o_scan_tmp = take(std::max(scan_temp_bytes(VP), tile_scan_temp_bytes((int)tiles)));
   p->o_rgbs = take(VP * 12);
   p->o_drgbs = take(VP * 16);  // [V,P,4]: dL/drgb (xyz) and the subdivision priority (w)
   // the instance arrays also serve the one-time sort of the 8P rank keys
@@ -591,7 +671,8 @@ int svr_batch_plan_create(int n_views, const svr_camera* cams, int64_t P, int64_
   p->o_kb = take(kv * 8);
   p->o_va = take(kv * 4);
   p->o_vb = take(kv * 4);
-  p->o_sort_tmp = take(std::max(sort_temp_bytes(kv), seg_sort_temp_bytes(p->cap, (int)tiles)));
+  p->o_sort_tmp = take(std::max({sort_temp_bytes(kv), seg_sort_temp_bytes(p->cap, (int)tiles),
+                                 tile_sort_temp_bytes(p->cap, (int)tiles)}));
   p->o_ranges = take((size_t)tiles * 8);
   p->o_tile_last = take((size_t)tiles * 4);
   p->o_ncontrib = take((size_t)pix * 4);
@@ -601,6 +682,7 @@ int svr_batch_plan_create(int n_views, const svr_camera* cams, int64_t P, int64_
   p->o_order_bwd = take((size_t)tiles * 4);
   p->o_order_tmp = take(sort_temp_bytes((size_t)tiles));
   p->o_pos = take((size_t)(8 * P) * 4);
+  p->o_valpos = take((size_t)(8 * P) * 4);
   p->bytes = align_up(off) + kAlign;
   p->order_flags = 3;
   p->fwd_ctas_per_sm = 0;
@@ -735,7 +817,8 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
   BatchPtrs q = ptrs(p, ws);
   const int P = (int)p->P;
   const size_t VP = (size_t)p->V * p->P;
-  cudaMemsetAsync(q.header, 0, kHeaderWords * sizeof(uint32_t), stream);
+  cudaMemsetAsync(q.header, 0, (kHeaderWords + (size_t)p->total_tiles) * sizeof(uint32_t), stream);
+  uint32_t* counts = p->binning ? q.counts : nullptr;
   const dim3 pgrid((P + 127) / 128);
   const int level_low = (p->rank_bits == kRankBits) ? 0 : kRankBits - (p->rank_bits - 3);  // 3*(16-L)
   const int tight = p->culling < 0 ? !p->exact : p->culling;
@@ -743,12 +826,12 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
   if (sh_bf16)                                                                                                \
     project_sh_kernel<D, __nv_bfloat16><<<pgrid, 128, 0, stream>>>(                                           \
         p->vt, P, vox_centers, vox_lengths, (const __nv_bfloat16*)sh0, (const __nv_bfloat16*)shs, M,         \
-        octree_paths, level_low, tight, q.ndup, q.bbox, q.quad, q.rgbs, q.header + 1, coverage_words(q));     \
+        octree_paths, level_low, tight, q.ndup, q.bbox, q.quad, q.rgbs, q.header + 1, coverage_words(q), counts); \
   else                                                                                                        \
     project_sh_kernel<D, float><<<pgrid, 128, 0, stream>>>(p->vt, P, vox_centers, vox_lengths,               \
                                                            (const float*)sh0, (const float*)shs, M,          \
                                                            octree_paths, level_low, tight, q.ndup, q.bbox,   \
-                                                           q.quad, q.rgbs, q.header + 1, coverage_words(q));
+                                                           q.quad, q.rgbs, q.header + 1, coverage_words(q), counts);
   const dim3 grid((P + 255) / 256, p->V);
   switch (sh_degree) {
     case 0: SVR_PROJ(0) break;
@@ -757,13 +840,8 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
     default: SVR_PROJ(3) break;
   }
 #undef SVR_PROJ
-  launch_scan_inclusive(q.ndup, q.scan, VP, q.scan_tmp, q.header, (unsigned long long)p->cap, q.header + 1, stream);
-  uint32_t* segs = q.header + 16;
-  group_segments_kernel<<<1, 64, 0, stream>>>(p->gt, P, q.scan, (uint32_t)p->cap, segs);
-  // the counting sort writes every tile's range itself; otherwise (radix
-  // grouping, or no instance capacity yet) empty tiles keep (0, 0)
-  if (!p->binning || p->cap == 0) cudaMemsetAsync(q.ranges, 0, (size_t)p->total_tiles * sizeof(uint2), stream);
-  if (!p->pos_ready || p->pos_paths != octree_paths) {
+  // (counting alone, as capacity fitting does, needs no positions)
+  if (p->cap > 0 && (!p->pos_ready || p->pos_paths != octree_paths)) {
     // Rank positions of all (voxel, quadrant) pairs: one stable radix sort of
     // the 8P compressed ranks in the (still free) instance arrays.
     const size_t n8 = 8 * (size_t)P;
@@ -771,48 +849,46 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
                                                                           q.header + 5);
     const int in_b = launch_radix_sort(q.ka, q.va, q.kb, q.vb, nullptr, q.header + 5, (uint32_t)n8, p->rank_bits,
                                        q.sort_tmp, stream);
-    rank_pos_scatter_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(n8, in_b ? q.vb : q.va, q.rank_pos);
+    rank_pos_scatter_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(n8, in_b ? q.vb : q.va, q.rank_pos, q.val_of_pos);
     p->pos_ready = true;
     p->pos_paths = octree_paths;
   }
+  if (p->binning) {
+    // Counting sort by tile: the projection's counts to ranges, every instance's
+    // rank position scattered into its tile's range, each range sorted.
+    uint32_t* keys = reinterpret_cast<uint32_t*>(q.ka);
+    launch_tile_ranges_from_counts(q.counts, (int)p->total_tiles, (uint32_t)p->cap, q.ranges, q.header, q.header + 1,
+                                   q.scan_tmp, q.sort_tmp, q.header + 6, stream);
+    if (p->cap > 0) {
+      scatter_positions_kernel<<<grid, 256, 0, stream>>>(p->vt, P, q.rank_pos, q.bbox, q.quad, q.counts, keys,
+                                                         (uint32_t)p->cap);
+      launch_tile_sort(q.ranges, (int)p->total_tiles, keys, q.val_of_pos, q.vb, p->cap, q.sort_tmp, q.header + 6,
+                       stream);
+    }
+    return check_last();
+  }
+  launch_scan_inclusive(q.ndup, q.scan, VP, q.scan_tmp, q.header, (unsigned long long)p->cap, q.header + 1, stream);
+  cudaMemsetAsync(q.ranges, 0, (size_t)p->total_tiles * sizeof(uint2), stream);
   if (p->cap > 0) {
     // Two-level sort: LSD radix passes over the tile bits only put every
-    // tile's instances together in generation order (ending in ka/va) -- or,
-    // with binning on, a counting sort by tile puts them together in no
-    // particular order -- then one CTA per tile sorts its segment by the
-    // rank-position bits into kb/vb.  Rank positions are unique inside a
-    // tile, so either way the result is the order of one stable sort by the
-    // full key.
+    // tile's instances together in generation order (ending in ka/va), then
+    // one CTA per tile sorts its segment by the rank-position bits into kb/vb.
+    uint32_t* segs = q.header + 16;
+    group_segments_kernel<<<1, 64, 0, stream>>>(p->gt, P, q.scan, (uint32_t)p->cap, segs);
     const bool odd = (sort_passes(p->key_bits - kPosShift) & 1) != 0;
     uint64_t* k0 = odd ? q.kb : q.ka;
     uint32_t* v0 = odd ? q.vb : q.va;
     uint64_t* k1 = odd ? q.ka : q.kb;
     uint32_t* v1 = odd ? q.va : q.vb;
-    if (p->binning) {
-      // Counting sort by tile instead: per-tile counts, their scan, then
-      // every instance scattered into its tile's range (in ka/va directly).
-      const uint32_t T = (uint32_t)p->total_tiles;
-      cudaMemsetAsync(q.oval, 0, (size_t)T * sizeof(uint32_t), stream);
-      duplicate_batch_kernel<kDupCount><<<grid, 256, 0, stream>>>(p->vt, P, q.rank_pos, q.bbox, q.quad, q.ndup,
-                                                                  q.scan, q.ka, q.va, (uint32_t)p->cap, q.header + 1,
-                                                                  q.oval, q.ranges);
-      launch_scan_inclusive(q.oval, q.order_fwd, T, q.scan_tmp, q.header + 6, ~0ull, nullptr, stream);
-      bin_ranges_kernel<<<(T + 255) / 256, 256, 0, stream>>>(T, q.oval, q.order_fwd, q.ranges);
-      duplicate_batch_kernel<kDupScatter><<<grid, 256, 0, stream>>>(p->vt, P, q.rank_pos, q.bbox, q.quad, q.ndup,
-                                                                    q.scan, q.ka, q.va, (uint32_t)p->cap,
-                                                                    q.header + 1, q.oval, q.ranges);
-    } else {
-      duplicate_batch_kernel<kDupWrite><<<grid, 256, 0, stream>>>(p->vt, P, q.rank_pos, q.bbox, q.quad, q.ndup,
-                                                                  q.scan, k0, v0, (uint32_t)p->cap, q.header + 1,
-                                                                  nullptr, nullptr);
-      for (int g = 0; g < p->gt.n; ++g) {
-        launch_radix_sort(k0, v0, k1, v1, segs + 2 * g, segs + 2 * g + 1, (uint32_t)p->cap, p->key_bits,
-                          q.sort_tmp, stream, kPosShift);
-        const uint32_t g_tiles = (g + 1 < p->gt.n ? p->gt.tile_base[g + 1] : (uint32_t)p->total_tiles) -
-                                 p->gt.tile_base[g];
-        launch_tile_ranges(q.ka, segs + 2 * g, segs + 2 * g + 1, (uint32_t)p->cap, kPosShift, p->gt.tile_base[g],
-                           g_tiles, q.ranges, stream);
-      }
+    duplicate_batch_kernel<<<grid, 256, 0, stream>>>(p->vt, P, q.rank_pos, q.bbox, q.quad, q.ndup, q.scan, k0, v0,
+                                                     (uint32_t)p->cap, q.header + 1);
+    for (int g = 0; g < p->gt.n; ++g) {
+      launch_radix_sort(k0, v0, k1, v1, segs + 2 * g, segs + 2 * g + 1, (uint32_t)p->cap, p->key_bits,
+                        q.sort_tmp, stream, kPosShift);
+      const uint32_t g_tiles = (g + 1 < p->gt.n ? p->gt.tile_base[g + 1] : (uint32_t)p->total_tiles) -
+                               p->gt.tile_base[g];
+      launch_tile_ranges(q.ka, segs + 2 * g, segs + 2 * g + 1, (uint32_t)p->cap, kPosShift, p->gt.tile_base[g],
+                         g_tiles, q.ranges, stream);
     }
     // the radix histograms in sort_tmp are dead here; the segment sort reuses it
     launch_tile_segment_sort(q.ranges, (int)p->total_tiles, q.ka, q.va, q.kb, q.vb, p->pos_bits, p->cap,
@@ -830,7 +906,8 @@ static int batch_render(svr_batch_plan* p, void* ws, VoxelArrays va, float* out_
   va.rgbs = q.rgbs;
   FwdTileOut out{q.tile_last, q.ncontrib, out_color, nullptr, nullptr, out_T, nullptr};
   const bool ordered = (p->order_flags & 1) != 0;
-  if (ordered) build_tile_order(p, q, nullptr, q.order_fwd, stream);
+  if (ordered) build_tile_order(p, q, nullptr, q.order_fwd, q.header + 2, stream);
+  else cudaMemsetAsync(q.header + 2, 0, sizeof(uint32_t), stream);
   launch_render_fwd_batch(p->vt, (int)p->total_tiles, q.ranges, p->cap > 0 ? q.vb : nullptr, va, (int)p->P,
                           (size_t)p->P * 3, out, p->n_samp, p->tile_size, p->stage, !p->exact, p->pair,
                           ordered ? q.order_fwd : nullptr, q.header + 2, p->fwd_ctas_per_sm, stream);
@@ -847,7 +924,8 @@ static int batch_backward(svr_batch_plan* p, void* ws, VoxelArrays va, const flo
   out.dL_drgbs = q.drgbs;
   out.err = q.header + 1;
   const bool ordered = (p->order_flags & 2) != 0;
-  if (ordered) build_tile_order(p, q, q.tile_last, q.order_bwd, stream);
+  if (ordered) build_tile_order(p, q, q.tile_last, q.order_bwd, q.header + 3, stream);
+  else cudaMemsetAsync(q.header + 3, 0, sizeof(uint32_t), stream);
   launch_render_bwd_batch(p->vt, (int)p->total_tiles, q.ranges, q.tile_last, p->cap > 0 ? q.vb : nullptr, va,
                           (int)p->P, (size_t)p->P * 3, (size_t)p->P * 4, in, out, p->n_samp, p->tile_size,
                           p->stage_bwd, !p->exact, p->pair_bwd < 0 ? p->pair : p->pair_bwd,

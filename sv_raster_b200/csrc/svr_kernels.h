@@ -68,6 +68,25 @@ void launch_tile_order(const uint2* ranges, const uint32_t* tile_last, uint32_t 
 void launch_tile_ranges(const uint64_t* keys, const uint32_t* d_start, const uint32_t* d_n, uint32_t cap,
                         int rank_bits, uint32_t tile_base, uint32_t n_tiles, uint2* ranges, cudaStream_t stream);
 
+// svr_tilesort.cu: the batched path's binning by 32-bit rank positions.
+// counts[n_tiles] become the scatter cursors; n_runs is one device word, zero at
+// the call; scan_temp and run_list hold tile_scan_temp_bytes / tile_sort_temp_bytes.
+size_t tile_scan_temp_bytes(int n_tiles);
+size_t tile_sort_temp_bytes(size_t cap, int n_tiles);
+void launch_tile_ranges_from_counts(uint32_t* counts, int n_tiles, uint32_t cap, uint2* ranges, uint32_t* d_total,
+                                    uint32_t* err, void* scan_temp, void* run_list, uint32_t* n_runs,
+                                    cudaStream_t stream);
+// Sorts every tile's rank positions [ranges[t].x, ranges[t].y) of `keys` (used as
+// scratch) and writes their values, val_of_pos[position], to the same places of
+// vals.
+void launch_tile_sort(const uint2* ranges, int n_tiles, uint32_t* keys, const uint32_t* val_of_pos, uint32_t* vals,
+                      size_t cap, const void* run_list, const uint32_t* n_runs, cudaStream_t stream);
+// launch_tile_order's order (ties aside) for few tiles in one launch, which also
+// zeroes the work counter.
+bool small_tile_order_fits(uint32_t n_tiles);
+void launch_small_tile_order(const uint2* ranges, const uint32_t* tile_last, uint32_t n_tiles, uint32_t* order,
+                             uint32_t* counter, cudaStream_t stream);
+
 // svr_render_fwd.cu / svr_render_bwd.cu
 // Plain one-view launches over the reference's 16x16 tile lists: four 8x8
 // CTAs per list; CTA i renders quadrant i % 4 of list order[i / 4] (largest
@@ -77,7 +96,7 @@ void launch_render_fwd(const ViewParams& vp, const uint2* ranges, const uint32_t
                        const FwdTileOut& out, int ns, bool depth, bool dist, bool normal, bool maxw,
                        const uint32_t* order, cudaStream_t stream);
 // Multi-view forms (no depth / distortion / normal outputs): persistent
-// grids taking tiles from `counter` (zeroed here) in the order of `order`
+// grids taking tiles from `counter` (zero at the launch) in the order of `order`
 // (identity when null); ctas_per_sm caps the resident CTAs per SM (0 = as
 // many as fit).  (tile, stage) must satisfy batch_tile_supported.
 bool batch_pair_supported(int tile, int stage);

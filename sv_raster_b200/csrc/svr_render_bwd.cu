@@ -281,7 +281,6 @@ void launch_render_bwd_batch(const ViewTable& views, int n_items, const uint2* r
                              cudaStream_t stream) {
   if (n_items <= 0) return;
   ensure_bwd_batch_attributes();
-  cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream);
   BwdBatchArgs args{views, n_items, ranges, tile_last, vals, va, P, rgb_view_stride, drgb_view_stride, in, out,
                     order, counter, coverage, -1};
   // Two pixels per thread has one warp per tile walk the list with all lanes on

@@ -281,7 +281,6 @@ void launch_render_fwd_batch(const ViewTable& views, int n_items, const uint2* r
                              const uint32_t* order, uint32_t* counter, int ctas_per_sm, cudaStream_t stream) {
   if (n_items <= 0) return;
   ensure_fwd_batch_attributes();
-  cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream);
   const FwdBatchArgs args{views, n_items, ranges, vals, va, P, rgb_view_stride, out, order, counter};
   if (pair && batch_pair_supported(tile, stage)) {
     if (tile == 8 && stage == 32) launch_fwd_pair_cfg<PairCfg<8, 32>>(args, ns, fast, ctas_per_sm, stream);

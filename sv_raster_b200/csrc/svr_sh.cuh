@@ -22,6 +22,44 @@ __device__ __forceinline__ float ldf(const TS* p, size_t i) {
   else return p[i];
 }
 
+// A voxel's rest coefficients are a row of 3 (M - 1) values; the first
+// sh_row<DEG>() of them are in use at degree DEG.  Rows staged in shared memory
+// lie an odd number of words apart: a lane's walk over its own is conflict-free.
+template <int DEG>
+constexpr int sh_row() { return 3 * ((DEG + 1) * (DEG + 1) - 1); }
+template <int DEG>
+constexpr int sh_stride() { return sh_row<DEG>() | 1; }
+
+// The warp brings the rows of the lanes in `wanted` into rows[32][sh_stride]
+// (lane v's voxel is i): row after row, eight in flight at once, a lane taking
+// elements lane and lane + 32.
+template <int DEG, typename TS>
+__device__ __forceinline__ void stage_sh_rows(const TS* __restrict__ shs, int64_t i, int rest, uint32_t wanted,
+                                              float* rows, int lane) {
+  constexpr int ROW = sh_row<DEG>(), STRIDE = sh_stride<DEG>(), U = 8;
+  if constexpr (ROW > 0) {
+#pragma unroll 1
+    for (int v0 = 0; v0 < 32; v0 += U) {
+      if (!((wanted >> v0) & ((1u << U) - 1u))) continue;
+      float t[U][2];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const TS* row = shs + (size_t)__shfl_sync(0xffffffffu, i, v0 + u) * rest;
+        const bool in = (wanted >> (v0 + u)) & 1u;
+        t[u][0] = in && lane < ROW ? ldf(row, lane) : 0.f;
+        if (ROW > 32) t[u][1] = in && lane + 32 < ROW ? ldf(row, lane + 32) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float* d = rows + (v0 + u) * STRIDE;
+        if (lane < ROW) d[lane] = t[u][0];
+        if (ROW > 32 && lane + 32 < ROW) d[lane + 32] = t[u][1];
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // rgb of one channel `c`; `sh` points at the voxel's (M-1) x 3 rest coefficients.
 template <int DEG, typename TS>
 __device__ __forceinline__ float sh_channel(float x, float y, float z, float base0, const TS* sh, int c) {

@@ -23,17 +23,10 @@ namespace svr {
 // 32 voxels together instead, element after element through shared memory (row
 // strides are odd, so a lane's walk over its row is free of conflicts).  Voxels
 // with consecutive ids then make full-width accesses.  1.93M visible of 2M
-// voxels, degree 3, fp32: the evaluation 117 -> 111 us (its rows came through the
+// voxels, degree 3, fp32: the evaluation 117 -> 97 us (its rows came through the
 // L1 cache before), the backward 563 -> 86 us; the rows alone take 56 us at the
 // copy bandwidth.
 constexpr int kShThreads = 128;
-constexpr int kShUnroll = 8;
-
-// Row elements of degree DEG (the coefficients above it are not touched).
-template <int DEG>
-constexpr int sh_row() { return 3 * ((DEG + 1) * (DEG + 1) - 1); }
-template <int DEG>
-constexpr int sh_stride() { return sh_row<DEG>() | 1; }
 
 template <int DEG, typename TS>
 __global__ void __launch_bounds__(kShThreads)
@@ -48,30 +41,7 @@ sh_eval_kernel(int n_idx, int P, int M, const int64_t* __restrict__ idx, const f
   const bool on = tid < n;
   const int64_t i = on ? (n_idx != 0 ? idx[tid] : (int64_t)tid) : 0;
   float* rows = s_rows + (threadIdx.x & ~31) * STRIDE;
-  if (ROW > 0) {
-    const int n_here = min(32, n - (tid - lane));
-    const int rest = (M - 1) * 3;
-    // Row after row, kShUnroll of them in flight at once; a lane takes elements
-    // lane and lane + 32.
-#pragma unroll 1
-    for (int v0 = 0; v0 < 32; v0 += kShUnroll) {
-      float t[kShUnroll][2];
-#pragma unroll
-      for (int u = 0; u < kShUnroll; ++u) {
-        const TS* row = shs + (size_t)__shfl_sync(0xffffffffu, i, v0 + u) * rest;
-        const bool in = v0 + u < n_here;
-        t[u][0] = in && lane < ROW ? ldf(row, lane) : 0.f;
-        if (ROW > 32) t[u][1] = in && lane + 32 < ROW ? ldf(row, lane + 32) : 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < kShUnroll; ++u) {
-        float* d = rows + (v0 + u) * STRIDE;
-        if (lane < ROW) d[lane] = t[u][0];
-        if (ROW > 32 && lane + 32 < ROW) d[lane + 32] = t[u][1];
-      }
-    }
-    __syncwarp();
-  }
+  stage_sh_rows<DEG>(shs, i, (M - 1) * 3, __ballot_sync(0xffffffffu, on), rows, lane);
   if (!on) return;
   float dx = centers[3 * i + 0] - cam_pos[0];
   float dy = centers[3 * i + 1] - cam_pos[1];
