@@ -383,6 +383,10 @@ int svr_batch_backward_grid(svr_batch_plan* plan, void* workspace, const float* 
  * over views (overwritten; backward.cu:514 per view). */
 int svr_batch_sh_backward(svr_batch_plan* plan, void* workspace, const float* vox_centers, int sh_degree, int M,
                           float* dL_dsh0, float* dL_dshs, float* subdiv, void* stream);
+/* The same with the gradients as bf16 (out_bf16 = 1; 4-byte aligned), rounded
+ * from the fp32 sums, or fp32 (0). */
+int svr_batch_sh_backward_as(svr_batch_plan* plan, void* workspace, const float* vox_centers, int sh_degree, int M,
+                             void* dL_dsh0, void* dL_dshs, int out_bf16, float* subdiv, void* stream);
 
 #ifdef __cplusplus
 }

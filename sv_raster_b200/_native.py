@@ -112,6 +112,7 @@ _SIGS = {
     "svr_batch_render_grid": (c_int, [c_p, c_p, c_p, c_p, c_p, c_p, c_int, c_p, c_p, c_p]),
     "svr_batch_backward_grid": (c_int, [c_p, c_p, c_p, c_p, c_p, c_p, c_int, c_p, c_p, c_p, c_p, c_p]),
     "svr_batch_sh_backward": (c_int, [c_p, c_p, c_p, c_int, c_int, c_p, c_p, c_p, c_p]),
+    "svr_batch_sh_backward_as": (c_int, [c_p, c_p, c_p, c_int, c_int, c_p, c_p, c_int, c_p, c_p]),
 }
 
 _lib = None

@@ -277,10 +277,22 @@ class BatchedRasterizer:
 
     def backward_sh(self, sh_degree, M, dL_dsh0, dL_dshs, subdiv=None):
         """SH gradients (and the subdivision priority) summed over views, from
-        the colour gradients of the last backward_render (overwritten)."""
-        check(lib().svr_batch_sh_backward(self.plan, self._p(self.ws), self._p(self.centers), int(sh_degree), int(M),
-                                          self._p(dL_dsh0), self._p(dL_dshs) if dL_dshs.numel() else None,
-                                          self._p(subdiv), self._stream()), "batch_sh_backward")
+        the colour gradients of the last backward_render (overwritten): fp32,
+        or bf16 when dL_dsh0 and dL_dshs are (fp32 sums rounded once)."""
+        bf16 = dL_dsh0.dtype == torch.bfloat16
+        if bf16 != (dL_dshs.dtype == torch.bfloat16):
+            raise ValueError("dL_dsh0 and dL_dshs must share a dtype")
+        check(lib().svr_batch_sh_backward_as(self.plan, self._p(self.ws), self._p(self.centers), int(sh_degree),
+                                             int(M), self._p(dL_dsh0), self._p(dL_dshs) if dL_dshs.numel() else None,
+                                             int(bf16), self._p(subdiv), self._stream()), "batch_sh_backward")
+
+    def _sh_grads(self, sh_degree, M, dtype):
+        """backward_sh into new tensors of the coefficients' dtype."""
+        dt = torch.bfloat16 if dtype == torch.bfloat16 else torch.float32
+        dsh0 = torch.empty(self.P, 3, dtype=dt, device=self.dev)
+        dshs = torch.empty(self.P, M - 1, 3, dtype=dt, device=self.dev)
+        self.backward_sh(sh_degree, M, dsh0, dshs)
+        return dsh0.to(dtype), dshs.to(dtype)
 
     # -- views of the flat outputs ---------------------------------------------
     def split_color(self, flat):
@@ -332,8 +344,9 @@ class BatchedRender(torch.autograd.Function):
         r = ctx.raster
         if dL_dT is None:
             dL_dT = torch.zeros_like(T)
-        dgeo, _sub, dsh0, dshs = r.backward(geos, T, dL_dcolor.contiguous(), dL_dT.contiguous(), ctx.sh_degree, ctx.M)
-        return None, None, dgeo.to(geos.dtype), dsh0.to(ctx.sh_dtype), dshs.to(ctx.sh_dtype)
+        dgeo = torch.zeros(r.P, 8, device=r.dev)
+        r.backward_render(geos, T, dL_dcolor.contiguous(), dL_dT.contiguous(), dgeo)
+        return (None, None, dgeo.to(geos.dtype)) + r._sh_grads(ctx.sh_degree, ctx.M, ctx.sh_dtype)
 
 
 def gather_grid_geos(vox_key, grid_pts, out):
@@ -394,13 +407,10 @@ class GridBatchedRender(torch.autograd.Function):
         if dL_dT is None:
             dL_dT = torch.zeros_like(T)
         dgrid = torch.zeros(ctx.M_grid, dtype=torch.float32, device=T.device)
-        P, M = vox_key.shape[0], ctx.M
         if ctx.fused:
             r.backward_render_grid(vox_key, dens, T, dL_dcolor.contiguous(), dL_dT.contiguous(), dgrid)
-            dsh0 = torch.empty(P, 3, device=T.device)
-            dshs = torch.empty(P, M - 1, 3, device=T.device)
-            r.backward_sh(ctx.sh_degree, M, dsh0, dshs)
         else:
-            dgeo, _sub, dsh0, dshs = r.backward(dens, T, dL_dcolor.contiguous(), dL_dT.contiguous(), ctx.sh_degree, M)
+            dgeo = torch.zeros(r.P, 8, device=r.dev)
+            r.backward_render(dens, T, dL_dcolor.contiguous(), dL_dT.contiguous(), dgeo)
             scatter_grid_grad(vox_key, dgeo, dgrid)
-        return (None, None, None, dgrid.to(ctx.grid_dtype), dsh0.to(ctx.sh_dtype), dshs.to(ctx.sh_dtype), None)
+        return (None, None, None, dgrid.to(ctx.grid_dtype)) + r._sh_grads(ctx.sh_degree, ctx.M, ctx.sh_dtype) + (None,)
