@@ -66,7 +66,7 @@ def rasterize_preprocess(image_width, image_height, tan_fovx, tan_fovy, cx, cy, 
         raise RuntimeError("vox_centers must have dimensions (num_points, 3)")
     dev = _cuda(vox_centers, "vox_centers").device
     P = vox_centers.size(0)
-    out_ndup = torch.zeros(P, dtype=torch.int32, device=dev)
+    out_ndup = torch.empty(P, dtype=torch.int32, device=dev)  # the projection writes every voxel's
     if P == 0:
         return out_ndup, torch.empty(0, dtype=torch.uint8, device=dev)
     L = lib()
@@ -116,10 +116,14 @@ def rasterize_voxels(n_samp_per_vox, image_width, image_height, tan_fovx, tan_fo
     P = vox_centers.size(0)
     H, W = int(image_height), int(image_width)
     fopt = dict(dtype=torch.float32, device=dev)
-    color = torch.zeros(3, H, W, **fopt)
-    depth = torch.zeros(3, H, W, **fopt) if (need_depth or need_distortion) else torch.empty(0)
-    normal = torch.zeros(3, H, W, **fopt) if need_normal else torch.empty(0)
-    T = torch.zeros(1, H, W, **fopt)
+    # compositing writes every pixel of the outputs that are asked for: zeros are
+    # for no voxels at all, and for the depth channels that are not
+    new = torch.zeros if P == 0 else torch.empty
+    color = new(3, H, W, **fopt)
+    all_depth = need_depth and need_distortion
+    depth = (new if all_depth else torch.zeros)(3, H, W, **fopt) if (need_depth or need_distortion) else torch.empty(0)
+    normal = new(3, H, W, **fopt) if need_normal else torch.empty(0)
+    T = new(1, H, W, **fopt)
     max_w = torch.zeros(P, 1, **fopt) if track_max_w else torch.empty(0)
     binning = torch.empty(0, dtype=torch.uint8, device=dev)
     L = lib()

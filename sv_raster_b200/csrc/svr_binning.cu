@@ -24,7 +24,7 @@
 namespace svr {
 
 // --------------------------------------------------------------------------
-// Inclusive scan of uint32 counts (three phases, no inter-CTA waiting)
+// Inclusive scan of uint32 counts (two phases, no inter-CTA waiting)
 // --------------------------------------------------------------------------
 // kScanThreads, kScanItems and kScanTile are declared in svr_kernels.h.
 size_t scan_temp_bytes(size_t n) {
@@ -47,36 +47,16 @@ scan_reduce_kernel(const uint32_t* __restrict__ in, size_t n, unsigned long long
   if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
 }
 
-// Single CTA: exclusive scan of the block sums (in place); writes the grand
-// total (clamped to 32 bits) and flags overflow of 32 bits or of `cap`.
-__global__ void __launch_bounds__(1024)
-scan_blocks_kernel(unsigned long long* __restrict__ block_sums, int nb, uint32_t* __restrict__ d_total,
-                   unsigned long long cap, uint32_t* __restrict__ err) {
-  __shared__ unsigned long long s_warp[1024 / 32 + 1];
-  unsigned long long running = 0;
-  for (int b0 = 0; b0 < nb; b0 += 1024) {
-    const int i = b0 + threadIdx.x;
-    const unsigned long long x = (i < nb) ? block_sums[i] : 0ull;
-    unsigned long long tot;
-    const unsigned long long ex = block_exclusive_scan<1024>(x, s_warp, tot);
-    if (i < nb) block_sums[i] = running + ex;
-    running += tot;
-  }
-  if (threadIdx.x == 0) {
-    if (running > 0xffffffffull) {
-      *d_total = 0xffffffffu;
-      if (err) atomicOr(err, SVR_DEVERR_CAPACITY);
-    } else {
-      *d_total = (uint32_t)running;
-      if (err && running > cap) atomicOr(err, SVR_DEVERR_CAPACITY);
-    }
-  }
-}
-
 __global__ void __launch_bounds__(kScanThreads)
-scan_apply_kernel(const uint32_t* __restrict__ in, size_t n, const unsigned long long* __restrict__ block_off,
-                  uint32_t* __restrict__ out) {
+scan_apply_kernel(const uint32_t* __restrict__ in, size_t n, const unsigned long long* __restrict__ block_sums,
+                  uint32_t* __restrict__ out, uint32_t* __restrict__ d_total, unsigned long long cap,
+                  uint32_t* __restrict__ err) {
   __shared__ unsigned long long s_warp[kScanThreads / 32 + 1];
+  // every CTA adds up the sums before its own (a few KB from the L2 cache) instead
+  // of a launch between the two that scans them
+  unsigned long long before = 0, offset;
+  for (unsigned b = threadIdx.x; b < blockIdx.x; b += kScanThreads) before += block_sums[b];
+  block_exclusive_scan<kScanThreads>(before, s_warp, offset);
   // Each thread owns kScanItems consecutive items: load through shared memory
   // so global accesses stay coalesced.
   __shared__ uint32_t s_val[kScanTile];
@@ -96,7 +76,7 @@ scan_apply_kernel(const uint32_t* __restrict__ in, size_t n, const unsigned long
     s += v[r];
   }
   unsigned long long tot;
-  unsigned long long run = block_exclusive_scan<kScanThreads>(s, s_warp, tot) + block_off[blockIdx.x];
+  unsigned long long run = block_exclusive_scan<kScanThreads>(s, s_warp, tot) + offset;
 #pragma unroll
   for (int r = 0; r < kScanItems; ++r) {
     run += v[r];
@@ -109,6 +89,12 @@ scan_apply_kernel(const uint32_t* __restrict__ in, size_t n, const unsigned long
     const size_t i = base + li;
     if (i < n) out[i] = s_val[li];
   }
+  // the last CTA has the total (clamped to 32 bits; past them or `cap` is flagged)
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    const unsigned long long total = offset + tot;
+    *d_total = (uint32_t)min(total, 0xffffffffull);
+    if (err && (total > 0xffffffffull || total > cap)) atomicOr(err, SVR_DEVERR_CAPACITY);
+  }
 }
 
 void launch_scan_inclusive(const uint32_t* in, uint32_t* out, size_t n, void* temp, uint32_t* d_total,
@@ -119,9 +105,8 @@ void launch_scan_inclusive(const uint32_t* in, uint32_t* out, size_t n, void* te
   }
   const int nb = (int)((n + kScanTile - 1) / kScanTile);
   unsigned long long* sums = reinterpret_cast<unsigned long long*>(temp);
-  scan_reduce_kernel<<<nb, kScanThreads, 0, stream>>>(in, n, sums);
-  scan_blocks_kernel<<<1, 1024, 0, stream>>>(sums, nb, d_total, cap, err);
-  scan_apply_kernel<<<nb, kScanThreads, 0, stream>>>(in, n, sums, out);
+  if (nb > 1) scan_reduce_kernel<<<nb - 1, kScanThreads, 0, stream>>>(in, n, sums);
+  scan_apply_kernel<<<nb, kScanThreads, 0, stream>>>(in, n, sums, out, d_total, cap, err);
 }
 
 // --------------------------------------------------------------------------

@@ -120,7 +120,7 @@ BinningLayout binning_layout(void* buf, size_t n, int n_tiles) {
 }
 
 // 21-level binning: the 16-level layout, then the wide keys' high halves
-// and the per-instance rank, tile and value arrays.
+// and the per-instance rank and value arrays.
 DeepBinning deep_layout(void* buf, size_t n, int n_tiles, size_t* bytes) {
   BinningLayout bl = binning_layout(buf, n, n_tiles);
   Carver c(buf ? static_cast<char*>(buf) + bl.bytes : nullptr);
@@ -130,11 +130,8 @@ DeepBinning deep_layout(void* buf, size_t n, int n_tiles, size_t* bytes) {
   d.vals_a = bl.vals_a;
   d.vals_b = bl.vals_b;
   d.sort_temp = bl.sort_temp;
-  d.vals_out = bl.vals_b;
-  d.keys_lo = bl.keys_b;
   d.keys_hi = c.take<uint64_t>(n);
   d.rank_of = c.take<uint64_t>(n);
-  d.tile_of = c.take<uint32_t>(n);
   d.val_of = c.take<uint32_t>(n);
   if (bytes) *bytes = bl.bytes + c.size();
   return d;
@@ -334,8 +331,11 @@ int svr_rasterize_render(const svr_camera* cam, int n_samp, int need_depth, int 
   FwdTileOut out{c.im.tile_last, c.im.n_contrib, out_color, out_depth, out_normal, out_T, max_w};
   const uint32_t n_tiles = (uint32_t)(c.vt.v[0].grid_x * c.vt.v[0].grid_y);
   cudaMemsetAsync(c.im.tile_last, 0, n_tiles * sizeof(uint32_t), stream);  // combined by atomicMax
-  launch_tile_order(c.im.ranges, nullptr, n_tiles, c.im.okey, c.im.oval, c.im.order, c.im.ocount, c.im.otemp,
-                    stream);
+  if (small_tile_order_fits(n_tiles))
+    launch_small_tile_order(c.im.ranges, nullptr, n_tiles, c.im.order, nullptr, stream);
+  else
+    launch_tile_order(c.im.ranges, nullptr, n_tiles, c.im.okey, c.im.oval, c.im.order, c.im.ocount, c.im.otemp,
+                      stream);
   launch_render_fwd(c.vt.v[0], c.im.ranges, c.n > 0 ? c.bl.vals_b : nullptr, va, out, n_samp, need_depth != 0,
                     need_distortion != 0, need_normal != 0, track_max_w != 0, c.im.order, stream);
   return check_launch(debug, stream);
@@ -448,9 +448,9 @@ int svr_binning_sorted_wide(const void* binning_buffer, int64_t num_rendered, in
   if (!binning_buffer || num_rendered < 0 || width <= 0 || height <= 0) return SVR_ERR_SHAPE;
   DeepBinning d = deep_layout(const_cast<void*>(binning_buffer), (size_t)num_rendered,
                               tiles_x(width) * tiles_y(height), nullptr);
-  if (keys_lo) *keys_lo = d.keys_lo;
+  if (keys_lo) *keys_lo = d.keys_b;
   if (keys_hi) *keys_hi = d.keys_hi;
-  if (vals) *vals = d.vals_out;
+  if (vals) *vals = d.vals_b;
   return SVR_OK;
 }
 

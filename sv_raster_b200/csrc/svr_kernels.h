@@ -82,7 +82,7 @@ void launch_tile_ranges_from_counts(uint32_t* counts, int n_tiles, uint32_t cap,
 void launch_tile_sort(const uint2* ranges, int n_tiles, uint32_t* keys, const uint32_t* val_of_pos, uint32_t* vals,
                       size_t cap, const void* run_list, const uint32_t* n_runs, cudaStream_t stream);
 // launch_tile_order's order (ties aside) for few tiles in one launch, which also
-// zeroes the work counter.
+// zeroes the work counter (unless null).
 bool small_tile_order_fits(uint32_t n_tiles);
 void launch_small_tile_order(const uint2* ranges, const uint32_t* tile_last, uint32_t n_tiles, uint32_t* order,
                              uint32_t* counter, cudaStream_t stream);
@@ -116,10 +116,10 @@ void launch_render_bwd_batch(const ViewTable& views, int n_items, const uint2* r
                              const BwdTileOut& out, int ns, int tile, int stage, bool fast, int pair,
                              const CoverageCount& coverage, const uint32_t* order, uint32_t* counter, int ctas_per_sm,
                              cudaStream_t stream);
-// svr_binning_deep.cu: binning of 21-level octrees (63-bit ranks).  The
-// sort pairs (keys_a, vals_a) / (keys_b, vals_b) and sort_temp are those of
-// the 16-level layout; vals_out / keys_lo are its sorted-value and sorted-key
-// arrays, keys_hi and the per-instance rank / tile / value arrays follow it.
+// svr_binning_deep.cu: binning of 21-level octrees (63-bit ranks).  The sort
+// pairs (keys_a, vals_a) / (keys_b, vals_b) and sort_temp are those of the
+// 16-level layout, and the results are left in the second (keys_b the wide keys'
+// low halves); keys_hi and the per-instance rank and value arrays follow it.
 struct DeepBinning {
   uint64_t* keys_a;
   uint64_t* keys_b;
@@ -127,10 +127,7 @@ struct DeepBinning {
   uint32_t* vals_b;
   void* sort_temp;
   uint64_t* rank_of;
-  uint32_t* tile_of;
   uint32_t* val_of;
-  uint32_t* vals_out;
-  uint64_t* keys_lo;
   uint64_t* keys_hi;
 };
 void launch_binning_deep(const ViewParams& vp, int P, const int64_t* octpaths, const uint2* bboxes,

@@ -334,7 +334,7 @@ small_tile_order_kernel(const uint2* __restrict__ ranges, const uint32_t* __rest
   __shared__ uint32_t s_at[256];
   __shared__ uint32_t s_warp[kOrderT / 32 + 1];
   const uint32_t tid = threadIdx.x, lane = tid & 31;
-  if (tid == 0) *counter = 0u;
+  if (tid == 0 && counter) *counter = 0u;
   if (tid < 256) s_at[tid] = 0u;
   __syncthreads();
   const auto bucket = [&](uint32_t t) {
