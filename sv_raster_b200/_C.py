@@ -12,21 +12,15 @@ import ctypes
 import torch
 
 from . import _native
-from ._native import Camera, check, lib
+from ._native import Camera, check, lib, on_device
+from ._native import ptr as _ptr
+from ._native import raw_stream as _stream
 
 MAX_NUM_LEVELS = 16   # config.h:16
 STEP_SZ_SCALE = 100.0  # config.h:21
 MAX_N_SAMP = 3         # config.h:23
 
 TILE = 16
-
-
-def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if (t is not None and t.numel() > 0) else ctypes.c_void_p(0)
-
-
-def _stream(dev):
-    return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
 
 
 def _f32(t, name):
@@ -70,7 +64,7 @@ def rasterize_preprocess(image_width, image_height, tan_fovx, tan_fovy, cx, cy, 
     if P == 0:
         return out_ndup, torch.empty(0, dtype=torch.uint8, device=dev)
     L = lib()
-    with torch.cuda.device(dev):
+    with on_device(dev):
         vc = _f32(vox_centers, "vox_centers")
         vl = _f32(vox_lengths, "vox_lengths")
         w2c = _mat(w2c_matrix, "w2c_matrix", dev)
@@ -130,7 +124,7 @@ def rasterize_voxels(n_samp_per_vox, image_width, image_height, tan_fovx, tan_fo
     img = torch.empty(L.svr_image_buffer_bytes(W, H), dtype=torch.uint8, device=dev)
     if P == 0:
         return 0, binning, img, color, depth, normal, T, max_w
-    with torch.cuda.device(dev):
+    with on_device(dev):
         num_rendered = geom_num_rendered(geomBuffer)  # host sync, as forward.cu:653
         if num_rendered == 0xFFFFFFFF:
             raise RuntimeError("rasterize_voxels: instance count overflows 32 bits")
@@ -185,7 +179,7 @@ def rasterize_voxels_backward(R, n_samp_per_vox, image_width, image_height, tan_
     subdiv = torch.zeros(P, 1, **fopt)
     need_dist = lambda_dist > 0
     L = lib()
-    with torch.cuda.device(dev):
+    with on_device(dev):
         vc = _f32(vox_centers, "vox_centers")
         vl = _f32(vox_lengths, "vox_lengths")
         g = _f32(geos, "geos")
@@ -220,7 +214,7 @@ def unpack_ImageState(image_width, image_height, imageBuffer):
     ranges = torch.zeros(ty, tx, 2, dtype=torch.int32, device=dev)
     tile_last = torch.zeros(ty, tx, dtype=torch.int32, device=dev)
     n_contrib = torch.zeros(H, W, dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib().svr_unpack_image_state(W, H, _ptr(imageBuffer), _ptr(ranges), _ptr(tile_last), _ptr(n_contrib),
                                           _stream(dev))
     check(st, "unpack_ImageState")
@@ -282,7 +276,7 @@ def sh_compute(D, indices, vox_centers, cam_pos, sh0, shs):
     rgbs = torch.zeros(P, 3, dtype=torch.float32, device=dev)
     if P == 0:
         return rgbs
-    with torch.cuda.device(dev):
+    with on_device(dev):
         vc = _f32(vox_centers, "vox_centers")
         cp = _f32(cam_pos, "cam_pos").to(dev)
         bf16 = sh0.dtype == torch.bfloat16
@@ -306,7 +300,7 @@ def sh_compute_bw(D, M, indices, vox_centers, cam_pos, rgbs, dL_drgbs):
     dL_dshs = torch.zeros(P, M - 1, 3, dtype=torch.float32, device=dev)
     if P == 0:
         return dL_dsh0, dL_dshs
-    with torch.cuda.device(dev):
+    with on_device(dev):
         vc = _f32(vox_centers, "vox_centers")
         cp = _f32(cam_pos, "cam_pos").to(dev)
         g = _f32(dL_drgbs, "dL_drgbs")
@@ -330,7 +324,7 @@ def unbiased_adam_step(sparse, param, grad, exp_avg, exp_avg_sq, step, lr, beta1
     """adam_step.cu:106-135 (in place)."""
     _adam_tensors(param, grad, exp_avg, exp_avg_sq)
     dev = param.device
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib().svr_unbiased_adam_step(int(bool(sparse)), param.numel(), _ptr(param), _ptr(grad), _ptr(exp_avg),
                                           _ptr(exp_avg_sq), float(step), float(lr), float(beta1), float(beta2),
                                           float(eps), _stream(dev))
@@ -341,7 +335,7 @@ def biased_adam_step(sparse, param, grad, exp_avg, exp_avg_sq, lr, beta1, beta2,
     """adam_step.cu:137-158 (in place)."""
     _adam_tensors(param, grad, exp_avg, exp_avg_sq)
     dev = param.device
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib().svr_biased_adam_step(int(bool(sparse)), param.numel(), _ptr(param), _ptr(grad), _ptr(exp_avg),
                                         _ptr(exp_avg_sq), float(lr), float(beta1), float(beta2), float(eps),
                                         _stream(dev))
@@ -353,7 +347,7 @@ def gather_triinterp_geo_params(vox_key, care_idx, grid_pts):
     dev = _cuda(grid_pts, "grid_pts").device
     n_vox = vox_key.size(0)
     out = torch.empty(n_vox, 8, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib().svr_gather_grid_params(1, care_idx.size(0), _ptr(_i64(vox_key, "vox_key")),
                                           _ptr(_i64(care_idx, "care_idx")), _ptr(_f32(grid_pts, "grid_pts")),
                                           _ptr(out), _stream(dev))
@@ -365,7 +359,7 @@ def gather_triinterp_geo_params_bw(vox_key, care_idx, num_grid_pts, dL_dgeo_para
     """geo_params_gather.cu:154-172 -> dL_dgrid_pts [M,1]."""
     dev = _cuda(dL_dgeo_params, "dL_dgeo_params").device
     out = torch.zeros(int(num_grid_pts), 1, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib().svr_gather_grid_params_bw(1, care_idx.size(0), _ptr(_i64(vox_key, "vox_key")),
                                              _ptr(_i64(care_idx, "care_idx")),
                                              _ptr(_f32(dL_dgeo_params, "dL_dgeo_params")), _ptr(out), _stream(dev))
@@ -379,7 +373,7 @@ def gather_triinterp_feat_params(vox_key, care_idx, grid_pts):
         raise RuntimeError("Only support n_dim=3 now.")
     dev = _cuda(grid_pts, "grid_pts").device
     out = torch.empty(vox_key.size(0), 8, 3, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib().svr_gather_grid_params(3, care_idx.size(0), _ptr(_i64(vox_key, "vox_key")),
                                           _ptr(_i64(care_idx, "care_idx")), _ptr(_f32(grid_pts, "grid_pts")),
                                           _ptr(out), _stream(dev))
@@ -393,7 +387,7 @@ def gather_triinterp_feat_params_bw(vox_key, care_idx, num_grid_pts, dL_dfeat_pa
         raise RuntimeError("Only support n_dim=3")
     dev = _cuda(dL_dfeat_params, "dL_dfeat_params").device
     out = torch.zeros(int(num_grid_pts), 3, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib().svr_gather_grid_params_bw(3, care_idx.size(0), _ptr(_i64(vox_key, "vox_key")),
                                              _ptr(_i64(care_idx, "care_idx")),
                                              _ptr(_f32(dL_dfeat_params, "dL_dfeat_params")), _ptr(out),

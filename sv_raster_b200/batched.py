@@ -12,7 +12,7 @@ import math
 
 import torch
 
-from ._native import Camera, check, lib
+from ._native import Camera, check, lib, raw_stream
 
 TILE = 16
 
@@ -191,10 +191,10 @@ class BatchedRasterizer:
             pass
 
     def _stream(self):
-        return ctypes.c_void_p(torch.cuda.current_stream(self.dev).cuda_stream)
+        return raw_stream(self.dev)
 
     def _p(self, t):
-        return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+        return t.data_ptr() if t is not None else None
 
     def header(self):
         """(total instance count, device error word) -- synchronises."""
@@ -352,21 +352,17 @@ class BatchedRender(torch.autograd.Function):
 def gather_grid_geos(vox_key, grid_pts, out):
     """out[p, c] = grid_pts[vox_key[p, c]] for every voxel (GatherGeoParams
     with all voxels cared for; grid and out fp32 or bf16)."""
-    P = vox_key.shape[0]
-    check(lib().svr_gather_grid_geo_all(P, ctypes.c_void_p(vox_key.data_ptr()), ctypes.c_void_p(grid_pts.data_ptr()),
-                                        int(grid_pts.dtype == torch.bfloat16), ctypes.c_void_p(out.data_ptr()),
-                                        int(out.dtype == torch.bfloat16),
-                                        ctypes.c_void_p(torch.cuda.current_stream(out.device).cuda_stream)),
+    check(lib().svr_gather_grid_geo_all(vox_key.shape[0], vox_key.data_ptr(), grid_pts.data_ptr(),
+                                        int(grid_pts.dtype == torch.bfloat16), out.data_ptr(),
+                                        int(out.dtype == torch.bfloat16), raw_stream(out.device)),
           "gather_grid_geo_all")
     return out
 
 
 def scatter_grid_grad(vox_key, dL_dgeos, dL_dgrid):
     """dL_dgrid[vox_key[p, c]] += dL_dgeos[p, c] (fp32) for every voxel."""
-    P = vox_key.shape[0]
-    check(lib().svr_scatter_grid_geo_all(P, ctypes.c_void_p(vox_key.data_ptr()), ctypes.c_void_p(dL_dgeos.data_ptr()),
-                                         ctypes.c_void_p(dL_dgrid.data_ptr()),
-                                         ctypes.c_void_p(torch.cuda.current_stream(dL_dgrid.device).cuda_stream)),
+    check(lib().svr_scatter_grid_geo_all(vox_key.shape[0], vox_key.data_ptr(), dL_dgeos.data_ptr(),
+                                         dL_dgrid.data_ptr(), raw_stream(dL_dgrid.device)),
           "scatter_grid_geo_all")
     return dL_dgrid
 

@@ -1,10 +1,8 @@
 """Total-variation gradient on grid points, interface of
 ``svraster_cuda.grid_loss_bw`` (backends/cuda/svraster_cuda/grid_loss_bw.py)."""
-import ctypes
-
 import torch
 
-from ._native import check, lib
+from ._native import check, lib, on_device, raw_stream
 
 
 def total_variation(grid_pts, vox_key, weight, vox_size_inv, no_tv_s, tv_sparse, grid_pts_grad):
@@ -21,9 +19,9 @@ def total_variation(grid_pts, vox_key, weight, vox_size_inv, no_tv_s, tv_sparse,
     k = vox_key.contiguous().to(torch.int64)
     s = vox_size_inv.contiguous().float()
     scratch = torch.empty(N * C, dtype=torch.uint8, device=dev) if tv_sparse else None
-    p = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None
-    with torch.cuda.device(dev):
+    p = lambda t: t.data_ptr() if t is not None else None
+    with on_device(dev):
         st = lib().svr_total_variation_bw(p(g), p(k), float(weight), p(s), int(bool(no_tv_s)), int(bool(tv_sparse)),
                                           N, C, p(scratch), p(grid_pts_grad),
-                                          ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+                                          raw_stream(dev))
     check(st, "total_variation_bw")

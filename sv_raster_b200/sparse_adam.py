@@ -10,7 +10,7 @@ import ctypes
 import torch
 
 from . import _C
-from ._native import check, lib
+from ._native import check, lib, on_device, raw_stream
 
 
 class SparseAdam(torch.optim.Optimizer):
@@ -100,8 +100,8 @@ class FusedSparseAdam(SparseAdam):
             Nn = (ctypes.c_int64 * n)(*[c[0].numel() for c in chunk])
             S = (ctypes.c_double * n)(*[float(c[2]['step']) for c in chunk])
             LR = (ctypes.c_double * n)(*[float(c[3]) for c in chunk])
-            with torch.cuda.device(dev):
+            with on_device(dev):
                 st = lib().svr_fused_adam_step(n, int(bool(self.sparse)), P, B, G, M, V, Nn, S, LR,
                                                float(betas[0]), float(betas[1]), float(eps),
-                                               ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+                                               raw_stream(dev))
             check(st, "fused_adam_step")
