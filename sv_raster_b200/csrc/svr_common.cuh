@@ -112,6 +112,30 @@ __device__ __forceinline__ float min3_nan(float a, float b, float c) {
   return d;
 }
 
+// Two independent fp32 operations in one instruction, each rounded as by itself.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
+        "l"(reinterpret_cast<unsigned long long&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return d;
+}
+
 // Arithmetic of the compositing loops.  EXACT is the reference's own
 // operations (IEEE division, libdevice expf): contributor counts and images
 // come out bit-identical.  FAST uses the hardware exponential (exp2 with the
@@ -175,6 +199,7 @@ struct PixelRay {
   float ix, iy, iz;      // 1 / direction (+inf for a zero component, of either sign)
   float rd_norm_inv;     // 1 / |camera-space direction|
   uint32_t quad;         // octant of the direction
+  float sx, sy, sz;      // -1 where the direction is negative, else 1
 };
 
 // Y_FIRST: which product of the direction's two-term dot products is rounded
@@ -214,6 +239,9 @@ __device__ __forceinline__ PixelRay make_pixel_ray(float pixx, float pixy, int W
   r.iy = 1.f / (r.dy + 0.f);
   r.iz = 1.f / (r.dz + 0.f);
   r.quad = ray_quadrant(r.dx, r.dy, r.dz);
+  r.sx = r.dx < 0.f ? -1.f : 1.f;
+  r.sy = r.dy < 0.f ? -1.f : 1.f;
+  r.sz = r.dz < 0.f ? -1.f : 1.f;
   return r;
 }
 

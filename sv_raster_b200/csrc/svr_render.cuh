@@ -281,18 +281,32 @@ struct ListReader {
 // Slab test (auxiliary.h:240-253) of a ray of the record's octant: the octant
 // says which plane of each slab comes first, so no minima of the two are
 // needed.  A ray in a slab's plane (0 * inf) gives NaN, which fails a <= b: it
-// misses, as with the minima.
+// misses, as with the minima.  Here and below x and y share an instruction where
+// both need the same operation (the forward of eight full-HD views: 6.34 -> 6.17
+// ms; the bits are the same).
 __device__ __forceinline__ float2 octant_ray_box(const float4& rel, const PixelRay& r) {
-  const float sx = (r.quad & 4u) ? -rel.w : rel.w, sy = (r.quad & 2u) ? -rel.w : rel.w,
-              sz = (r.quad & 1u) ? -rel.w : rel.w;
-  return make_float2(max3_nan((rel.x - sx) * r.ix, (rel.y - sy) * r.iy, (rel.z - sz) * r.iz),
-                     min3_nan((rel.x + sx) * r.ix, (rel.y + sy) * r.iy, (rel.z + sz) * r.iz));
+  const float2 half = make_float2(rel.w, rel.w), at = make_float2(rel.x, rel.y), inv = make_float2(r.ix, r.iy);
+  const float2 nr = mul2(fma2(make_float2(-r.sx, -r.sy), half, at), inv);
+  const float2 fr = mul2(fma2(make_float2(r.sx, r.sy), half, at), inv);
+  return make_float2(max3_nan(nr.x, nr.y, fmaf(-r.sz, rel.w, rel.z) * r.iz),
+                     min3_nan(fr.x, fr.y, fmaf(r.sz, rel.w, rel.z) * r.iz));
 }
 
 // The same from the two planes staged in crossing order.
 __device__ __forceinline__ float2 near_far_ray_box(const float4& nr, const float4& fr, const PixelRay& r) {
-  return make_float2(max3_nan(nr.x * r.ix, nr.y * r.iy, nr.z * r.iz),
-                     min3_nan(fr.x * r.ix, fr.y * r.iy, fr.z * r.iz));
+  const float2 inv = make_float2(r.ix, r.iy);
+  const float2 n2 = mul2(make_float2(nr.x, nr.y), inv), f2 = mul2(make_float2(fr.x, fr.y), inv);
+  return make_float2(max3_nan(n2.x, n2.y, nr.z * r.iz), min3_nan(f2.x, f2.y, fr.z * r.iz));
+}
+
+// Place in the unit cube of the point at t, from the voxel's corner (xyz) and 1/l.
+__device__ __forceinline__ void place_in_voxel(const PixelRay& r, float t, const float4& corner, float inv_l, float& qx,
+                                               float& qy, float& qz) {
+  const float2 at = fma2(make_float2(t, t), make_float2(r.dx, r.dy), make_float2(r.ox, r.oy));
+  const float2 q = mul2(add2(at, make_float2(-corner.x, -corner.y)), make_float2(inv_l, inv_l));
+  qx = q.x;
+  qy = q.y;
+  qz = (fmaf(t, r.dz, r.oz) - corner.z) * inv_l;
 }
 
 // Fast arithmetic: exp(-optical depth) of a segment from its samples' summed
@@ -315,10 +329,8 @@ __device__ __forceinline__ float record_transmittance(const FwdStage<SB>& s, int
   const float step_sz = (b - a) * (1.f / NS);
   const float stx = step_sz * ray.dx, sty = step_sz * ray.dy, stz = step_sz * ray.dz;
   const float t0 = a + 0.5f * step_sz;
-  const float ptx = ray.ox + t0 * ray.dx, pty = ray.oy + t0 * ray.dy, ptz = ray.oz + t0 * ray.dz;
-  float qx = (ptx - cr.x) * vox_l_inv;
-  float qy = (pty - cr.y) * vox_l_inv;
-  float qz = (ptz - cr.z) * vox_l_inv;
+  float qx, qy, qz;
+  place_in_voxel(ray, t0, cr, vox_l_inv, qx, qy, qz);
   const float qsx = stx * vox_l_inv, qsy = sty * vox_l_inv, qsz = stz * vox_l_inv;
 #pragma unroll
   for (int k = 0; k < NS; ++k) {

@@ -201,10 +201,8 @@ __device__ __forceinline__ bool pair_pixel_record(const PairRecord& rec, PairPix
   const float vox_l_inv = nr.w;
   const float step_sz = (b - a) * (1.f / NS);
   const float t0 = a + 0.5f * step_sz;
-  const float ptx = p.ray.ox + t0 * p.ray.dx, pty = p.ray.oy + t0 * p.ray.dy, ptz = p.ray.oz + t0 * p.ray.dz;
-  float qx = (ptx - cr.x) * vox_l_inv;
-  float qy = (pty - cr.y) * vox_l_inv;
-  float qz = (ptz - cr.z) * vox_l_inv;
+  float qx, qy, qz;
+  place_in_voxel(p.ray, t0, cr, vox_l_inv, qx, qy, qz);
   constexpr bool kSplit = FAST && NS == 1;
   float exp_neg, dd_dd = 0.f;  // one sample: d(optical depth)/d(density) at it
   float dI_dgeo[8];            // several samples: d(optical depth)/d(corner densities)
