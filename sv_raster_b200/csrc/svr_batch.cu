@@ -80,14 +80,34 @@ struct TileRect {
   }
 };
 
+// View-dependent colour of a visible voxel (sh_compute.cu:54-106); m holds the
+// view's w2c and c2w.
+template <int DEG, typename TS>
+__device__ __forceinline__ void view_colour(const float* m, float cx, float cy, float cz, const float c0[3],
+                                            const TS* sh, float* __restrict__ rgb) {
+  float dx = cx - m[12 + 3], dy = cy - m[12 + 7], dz = cz - m[12 + 11];
+  const float rn = rnorm3df(dx, dy, dz);
+  dx = dx * rn; dy = dy * rn; dz = dz * rn;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) rgb[c] = sh_channel<DEG>(dx, dy, dz, c0[c], sh, c);
+}
+
 // One thread per voxel, looping over the views: the voxel's centre and size are
 // read once and kept in registers, so each view costs the projection arithmetic
 // and the per-(view, voxel) writes only.
 // With `counts`, every visible pair also adds its instances to its tiles' counts
 // (a warp takes the pairs of many tiles together, one tile per lane): 1.78 -> 2.22
-// ms for 8M voxels and eight views, where counting in a pass of its own, which
+// ms (before SH_LAST) for 8M voxels and eight views, where counting in a pass of its own, which
 // re-read 20 bytes per pair, took 0.88.
-template <int DEG, typename TS>
+//
+// SH_LAST (two views and more): the colours follow all projections, with the
+// coefficients in registers, so they are read once for all views, all in flight
+// at once, and are not alive during the projections (where they cost half the
+// occupancy): 2.20 -> 1.96 ms for 8M voxels and eight views. With one view there
+// is nothing to share and the coefficients are read through the cache where they
+// are used: 123 us for 2M voxels, 142 with SH_LAST, 218 with the rows staged in
+// shared memory.
+template <int DEG, typename TS, bool SH_LAST>
 __global__ void __launch_bounds__(128)
 project_sh_kernel(const __grid_constant__ ViewTable views, int P, const float* __restrict__ centers,
                   const float* __restrict__ lengths, const TS* __restrict__ sh0, const TS* __restrict__ shs, int M,
@@ -111,13 +131,8 @@ project_sh_kernel(const __grid_constant__ ViewTable views, int P, const float* _
     atomicOr(err, SVR_DEVERR_LEVEL);
   const float cx = centers[3 * iv], cy = centers[3 * iv + 1], cz = centers[3 * iv + 2];
   const float len = lengths[iv];
-  // The rest coefficients are read per visible view through the cache: holding
-  // 45 of them in registers across the views cost the kernel half its occupancy,
-  // and staging the rows in shared memory was slower with one view (123 -> 218
-  // us, 2M voxels) and no faster with eight.
   const TS* sh = shs + iv * (M - 1) * 3;
-  float c0[3];
-  bool loaded = false;
+  unsigned long long seen = 0ull;  // the views that see this voxel
   for (int v = 0; v < views.n; ++v) {
     const size_t o = (size_t)v * P + iv;
     const float* m = s_m[v];
@@ -152,18 +167,24 @@ project_sh_kernel(const __grid_constant__ ViewTable views, int P, const float* _
       }
     }
     if (!visible) continue;
-    if (!loaded) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) c0[c] = ldf(sh0, 3 * iv + c);
-      loaded = true;
-    }
-    // View-dependent colour of this visible voxel (sh_compute.cu:54-106).
-    float dx = cx - m[12 + 3], dy = cy - m[12 + 7], dz = cz - m[12 + 11];
-    const float rn = rnorm3df(dx, dy, dz);
-    dx = dx * rn; dy = dy * rn; dz = dz * rn;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) rgbs[3 * o + c] = sh_channel<DEG>(dx, dy, dz, c0[c], sh, c);
     px += min((bb_xmax(pr.bbox) - bb_xmin(pr.bbox) + 1u) * (bb_ymax(pr.bbox) - bb_ymin(pr.bbox) + 1u), 1u << 20);
+    if constexpr (SH_LAST) {
+      seen |= 1ull << v;
+    } else {
+      const float c0[3] = {ldf(sh0, 3 * iv), ldf(sh0, 3 * iv + 1), ldf(sh0, 3 * iv + 2)};
+      view_colour<DEG>(m, cx, cy, cz, c0, sh, rgbs + 3 * o);
+    }
+  }
+  if (SH_LAST && seen) {
+    constexpr int ROW = sh_row<DEG>();
+    float row[ROW > 0 ? ROW : 1];
+#pragma unroll
+    for (int k = 0; k < ROW; ++k) row[k] = ldf(sh, k);
+    const float c0[3] = {ldf(sh0, 3 * iv), ldf(sh0, 3 * iv + 1), ldf(sh0, 3 * iv + 2)};
+    for (unsigned long long left = seen; left; left &= left - 1) {
+      const int v = __ffsll((long long)left) - 1;
+      view_colour<DEG>(s_m[v], cx, cy, cz, c0, row, rgbs + 3 * ((size_t)v * P + iv));
+    }
   }
   __syncwarp();
   px = __reduce_add_sync(0xffffffffu, px);
@@ -833,16 +854,18 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
   const dim3 pgrid((P + 127) / 128);
   const int level_low = (p->rank_bits == kRankBits) ? 0 : kRankBits - (p->rank_bits - 3);  // 3*(16-L)
   const int tight = p->culling < 0 ? !p->exact : p->culling;
+#define SVR_PROJ_AS(D, TS, LAST)                                                                              \
+  project_sh_kernel<D, TS, LAST><<<pgrid, 128, 0, stream>>>(                                                  \
+      p->vt, P, vox_centers, vox_lengths, (const TS*)sh0, (const TS*)shs, M, octree_paths, level_low, tight,  \
+      q.ndup, q.bbox, q.quad, q.rgbs, q.header + 1, coverage_words(q), counts)
 #define SVR_PROJ(D)                                                                                           \
-  if (sh_bf16)                                                                                                \
-    project_sh_kernel<D, __nv_bfloat16><<<pgrid, 128, 0, stream>>>(                                           \
-        p->vt, P, vox_centers, vox_lengths, (const __nv_bfloat16*)sh0, (const __nv_bfloat16*)shs, M,         \
-        octree_paths, level_low, tight, q.ndup, q.bbox, q.quad, q.rgbs, q.header + 1, coverage_words(q), counts); \
-  else                                                                                                        \
-    project_sh_kernel<D, float><<<pgrid, 128, 0, stream>>>(p->vt, P, vox_centers, vox_lengths,               \
-                                                           (const float*)sh0, (const float*)shs, M,          \
-                                                           octree_paths, level_low, tight, q.ndup, q.bbox,   \
-                                                           q.quad, q.rgbs, q.header + 1, coverage_words(q), counts);
+  if (sh_bf16) {                                                                                              \
+    if (p->V > 1) SVR_PROJ_AS(D, __nv_bfloat16, true);                                                        \
+    else SVR_PROJ_AS(D, __nv_bfloat16, false);                                                                \
+  } else {                                                                                                    \
+    if (p->V > 1) SVR_PROJ_AS(D, float, true);                                                                \
+    else SVR_PROJ_AS(D, float, false);                                                                        \
+  }
   const dim3 grid((P + 255) / 256, p->V);
   switch (sh_degree) {
     case 0: SVR_PROJ(0) break;
@@ -851,6 +874,7 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
     default: SVR_PROJ(3) break;
   }
 #undef SVR_PROJ
+#undef SVR_PROJ_AS
   // (counting alone, as capacity fitting does, needs no positions)
   if (p->cap > 0 && (!p->pos_ready || p->pos_paths != octree_paths)) {
     // Rank positions of all (voxel, quadrant) pairs: one stable radix sort of
