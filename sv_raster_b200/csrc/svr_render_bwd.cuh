@@ -220,8 +220,12 @@ __device__ __forceinline__ bool bwd_pixel_record(const FwdStage<SB>& s, int j, c
     const float step_sz = (b - a) * (1.f / NS);
     const float stx = step_sz * ray.dx, sty = step_sz * ray.dy, stz = step_sz * ray.dz;
     const float t0 = a + 0.5f * step_sz;
-    float qx, qy, qz;
-    place_in_voxel(ray, t0, cr, vox_l_inv, qx, qy, qz);
+    // Scalar here: with x and y packed, as the forward has it, this kernel took 883
+    // us against 872 for one 1297x840 view (the same values either way).
+    const float ptx = ray.ox + t0 * ray.dx, pty = ray.oy + t0 * ray.dy, ptz = ray.oz + t0 * ray.dz;
+    float qx = (ptx - cr.x) * vox_l_inv;
+    float qy = (pty - cr.y) * vox_l_inv;
+    float qz = (ptz - cr.z) * vox_l_inv;
     const float qsx = stx * vox_l_inv, qsy = sty * vox_l_inv, qsz = stz * vox_l_inv;
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
