@@ -207,3 +207,31 @@ def test_adam_remainders_and_misaligned_starts(n, offset, sparse, biased):
     want = O.adam(host[0], host[1], host[2], host[3], 5, 0.02, 0.9, 0.99, 1e-8, biased=biased, sparse=sparse, mode="f64")
     for a, w in zip(got, want):
         assert np.abs(a.cpu().numpy() - w).max() < 2e-6
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("sizes", [(1, 7, 4096), (8 << 20,), ((8 << 20) - 2, 3), ((8 << 20) + 2051, 5, 1023)])
+def test_fused_adam_equals_single_groups(sizes, dtype, sparse):
+    """Several groups in one launch, kept in the cache or streamed past it, with
+    remainders: the same bits as each group by itself (bf16: on the stored values,
+    rounded once)."""
+    from sv_raster_b200.sparse_adam import FusedSparseAdam, SparseAdam
+    gen = torch.Generator(device="cuda").manual_seed(sum(sizes))
+    draw = lambda n: torch.randn(n, device="cuda", generator=gen)
+    one = [draw(n).to(dtype).requires_grad_(True) for n in sizes]
+    ref = [p.detach().float().requires_grad_(True) for p in one]
+    for p, q in zip(one, ref):
+        g = draw(p.numel())
+        g[::3] = 0.0
+        g[: p.numel() // 2] = 0.0  # whole groups of four without a gradient
+        p.grad_dtype = torch.float32  # parameters in 16 bits keep their gradients in 32
+        p.grad, q.grad = g, g.clone()
+    a = FusedSparseAdam([{"params": [p], "lr": 0.01 * (k + 1)} for k, p in enumerate(one)], sparse=sparse)
+    b = SparseAdam([{"params": [q], "lr": 0.01 * (k + 1)} for k, q in enumerate(ref)], sparse=sparse)
+    a.step()
+    b.step()
+    for p, q in zip(one, ref):
+        assert torch.equal(p.detach(), q.detach().to(dtype))
+        assert torch.equal(a.state[p]["exp_avg"], b.state[q]["exp_avg"])
+        assert torch.equal(a.state[p]["exp_avg_sq"], b.state[q]["exp_avg_sq"])
