@@ -272,15 +272,17 @@ int svr_batch_plan_invalidate_geometry(svr_batch_plan* plan);
  * depend on the schedule (gradients only up to the order of floating-point
  * additions). */
 int svr_batch_plan_set_schedule(svr_batch_plan* plan, int order_flags, int fwd_ctas_per_sm, int bwd_ctas_per_sm);
-/* Segment-size buckets of the per-tile segment sort in svr_batch_prepare:
- * tiles of at most small_n (256, 512 or 1024) instances are sorted by one
+/* Segment-size buckets of the per-tile segment sort that follows the radix
+ * grouping (svr_batch_plan_set_binning 0; the counting sort has a tile sort of
+ * its own without them): tiles of at most small_n (256, 512 or 1024) instances are sorted by one
  * small CTA each, longer ones in runs of `chunk` (2048 or 4096) instances
  * merged afterwards.  Defaults 512 / 4096; the order is the same for all. */
 int svr_batch_plan_set_sort_buckets(svr_batch_plan* plan, int small_n, int chunk);
-/* How svr_batch_prepare groups the instances by tile before the per-tile
- * segment sort: 1 (default) a counting sort (per-tile counts, their scan,
- * one scatter pass with one atomic per tile per warp), 0 LSD radix passes
- * over the tile bits of the keys.  The sorted lists are the same for both. */
+/* How svr_batch_prepare sorts the instances by (tile, rank): 1 (default) a
+ * counting sort by tile (counts taken in the projection, their scan, one
+ * scatter of 32-bit rank positions) and a sort of each tile's positions, 0 LSD
+ * radix passes over the tile bits of 64-bit keys and a segment sort per tile.
+ * The sorted lists are the same for both. */
 int svr_batch_plan_set_binning(svr_batch_plan* plan, int binning);
 /* Records staged into shared memory per round by the compositing kernels:
  * 128, 256 (default) or 512 with 16x16 tiles, 32, 64 (default) or 128 with
@@ -319,15 +321,17 @@ int svr_batch_plan_set_arithmetic(svr_batch_plan* plan, int exact);
 int svr_batch_plan_set_culling(svr_batch_plan* plan, int culling);
 /* Pixels per thread of the compositing kernels: 1 (default) or 2 (a warp
  * covers an 8x8 block, each lane two pixels four rows apart; a record's
- * shared-memory fields are read once for both and, in the backward, one warp
- * reduction serves both).  Used with 8x8 tiles staging 32 or 64 records and
+ * shared-memory fields are read once for both and, in the backward, they share
+ * a gradient row).  Used with 8x8 tiles staging 32 or 64 records and
  * 16x16 tiles staging 128 or 256; other tile configurations run one pixel
- * per thread.  Images, T and contributor counts do not depend on it. */
+ * per thread, and so does the backward of fewer than 65,536 tiles or of records
+ * under 16 pixels per instance on average, which it is faster for.  Images, T
+ * and contributor counts do not depend on it. */
 int svr_batch_plan_set_pixels_per_thread(svr_batch_plan* plan, int pixels);
 /* Pixels per thread of svr_batch_backward alone: 1 or 2, or 0 to follow
  * svr_batch_plan_set_pixels_per_thread (default).  The forward walks each
- * pixel's own records with one pixel per thread, while the backward's warp
- * reduction favours two, so the best choices can differ. */
+ * pixel's own records with one pixel per thread; the backward walks a list with
+ * all lanes on one record with two, so the best choices can differ. */
 int svr_batch_plan_set_backward_pixels_per_thread(svr_batch_plan* plan, int pixels);
 int64_t svr_batch_plan_pixels(const svr_batch_plan* plan);
 int64_t svr_batch_plan_tiles(const svr_batch_plan* plan);

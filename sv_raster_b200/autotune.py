@@ -9,11 +9,11 @@ gradients agree up to the order of floating-point additions):
   (``BatchedRasterizer.set_schedule``; its cap on resident CTAs per SM can be
   searched too by listing ``(ordered, cap)`` pairs, but full occupancy won on
   every scene measured, so the default space leaves it out).
-* ``bin`` -- how instances are grouped by tile before the per-tile sort:
-  counting sort with atomics (1) or radix passes over the tile bits (0)
+* ``bin`` -- how instances are sorted by tile and rank: counting sort of rank
+  positions (1) or radix passes over the tile bits and a segment sort (0)
   (``BatchedRasterizer.set_binning``).
-* ``sort`` -- segment-size buckets of the per-tile segment sort: the largest
-  segment sorted by one small CTA and the chunk length of the chunked sort
+* ``sort`` -- segment-size buckets of the per-tile segment sort that follows the
+  radix passes (without effect on the counting sort): the largest segment sorted by one small CTA and the chunk length of the chunked sort
   (``BatchedRasterizer.set_sort_buckets``).
 * ``reduce`` -- ``set_reduction``'s argument, kept for choices saved with it
   (the backward has one gradient reduction for any number of lanes).
@@ -27,13 +27,12 @@ gradients agree up to the order of floating-point additions):
   both kernels with one depth, and the two kernels prefer different ones
   (c4: forward 64, backward 32 records).
 * ``ppt`` -- pixels per compositing thread, 1 or 2 (two pixels of an 8x8
-  warp block share each record's loads and, in the backward, its warp
-  reduction; ``BatchedRasterizer.set_pixels_per_thread``), timed with the
+  warp block share each record's loads; ``BatchedRasterizer.set_pixels_per_thread``), timed with the
   forward after the tile.
 * ``bppt`` -- the backward's own pixels per thread (0: as ``ppt``), timed
-  with the backward: the forward walks each pixel's own records, which two
-  pixels per thread cannot, while the backward's warp reduction favours two
-  (``set_backward_pixels_per_thread``).
+  with the backward: with two, a warp walks a tile's list with all lanes on one
+  record, which the backward takes where tiles are many and records broad (it
+  decides on the device) (``set_backward_pixels_per_thread``).
 * ``tile`` -- compositing tile size of the batched path (8, 16 or 32 pixels)
   with the voxel-staging depth (records staged into shared memory per round)
   (``BatchedRasterizer.set_tile_size``; the tile size changes the binning, so

@@ -96,9 +96,9 @@ class BatchedRasterizer:
             check(L.svr_batch_plan_set_backward_staging(plan, self.staging_bwd), "batch_plan_set_backward_staging")
 
     def set_binning(self, binning=1):
-        """How prepare groups the instances by tile before the per-tile sort:
-        1 a counting sort (counts, scan, atomic scatter), 0 radix passes over
-        the tile bits.  The sorted lists are the same."""
+        """How prepare sorts the instances by tile and rank: 1 a counting sort
+        (counts, scan, scatter of rank positions, tile sort), 0 radix passes
+        over the tile bits and a segment sort.  The sorted lists are the same."""
         check(lib().svr_batch_plan_set_binning(self.plan, int(binning)), "batch_plan_set_binning")
         self.binning = int(binning)
 
@@ -169,7 +169,8 @@ class BatchedRasterizer:
         self.staging_bwd = None if records is None else r
 
     def set_sort_buckets(self, small_n=512, chunk=4096):
-        """Segment-size buckets of the per-tile segment sort (small_n in
+        """Segment-size buckets of the per-tile segment sort after the radix
+        grouping (without effect on the counting sort; small_n in
         256/512/1024, chunk in 2048/4096); the sorted order is the same for all."""
         self.sort_buckets = (int(small_n), int(chunk))
         check(lib().svr_batch_plan_set_sort_buckets(self.plan, *self.sort_buckets), "batch_plan_set_sort_buckets")

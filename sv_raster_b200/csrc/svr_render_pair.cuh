@@ -5,10 +5,7 @@
 // (l & 7, l >> 3) and (l & 7, (l >> 3) + 4).  A staged record that a warp's
 // ballot selects is tested against both pixels; the records' shared-memory
 // fields are read once for the pair, and in the backward the two pixels'
-// gradients are added in registers before the one warp reduction of the
-// record.  With one pixel per thread the same 8x8 block is two warps, and a
-// record touching both halves costs two ballots, two sets of loads and two
-// reductions.
+// gradients are added in registers and take one row.
 //
 // The per-pixel arithmetic is the one of svr_render_fwd.cuh /
 // svr_render_bwd.cuh (forward.cu:182-316, backward.cu:246-418) without the

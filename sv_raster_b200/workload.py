@@ -59,6 +59,12 @@ def tune_raster(raster, geos, sh0, shs):
     return out
 
 
+def _order_launches(tiles):
+    """Launches of a tile work order: one for up to 6,144 tiles, else a key kernel and
+    one 3-kernel sort pass."""
+    return 1 if tiles <= 6144 else 4
+
+
 class _Timer:
     """CUDA-event timing of one kernel stage on the launching stream."""
 
@@ -173,9 +179,9 @@ class PlainWorkload:
         for cam, _, _ in self.cams:
             T_ = math.ceil(cam.width / 16) * math.ceil(cam.height / 16)
             passes = math.ceil(int(T_).bit_length() / 10)  # radix passes over the tile bits (8-10 bit digits)
-            # preprocess 1 + scan 3 + duplicate 1 + sort 3/pass + ranges 1 + segment sort 4
-            # + tile order (key kernel + one 3-kernel sort pass) 4 + fwd 1 + bwd 1 + sh 2
-            n += 1 + 3 + 1 + 3 * passes + 1 + 4 + 4 + 1 + 1 + 2
+            # preprocess 1 + scan 2 + duplicate 1 + sort 3/pass + ranges 1 + segment sort 4
+            # + tile order + fwd 1 + bwd 1 + sh 2
+            n += 1 + 2 + 1 + 3 * passes + 1 + 4 + _order_launches(T_) + 1 + 1 + 2
         return n
 
     def kernel_stats(self):
@@ -394,14 +400,16 @@ class BatchedWorkload:
         passes = math.ceil(int(T_).bit_length() / 10)  # radix passes over the tile bits (8-10 bit digits)
         g = self.raster.n_groups
         order = self.raster.schedule[0]
-        # project 1 + scan 3 + segments 1 + grouping by tile + segment sort 4 (plan, small,
-        # chunk, merge) + per ordered compositing stage a tile-order key kernel and one
-        # 3-kernel sort pass + fwd 1 + bwd 1 + sh 1.  Grouping by tile: counting sort =
-        # count 1 + tile scan 3 + ranges 1 + scatter 1; radix = duplicate 1 + (sort 3/pass
-        # + ranges 1) per group.
-        n_order = 4 * ((order & 1) + ((order >> 1) & 1))
-        grouping = 6 if getattr(self.raster, "binning", 0) else 1 + g * (3 * passes + 1)
-        return 1 + 3 + 1 + grouping + 4 + n_order + 1 + 1 + 1
+        # project 1 + grouping by tile and sort + per ordered compositing stage its tile
+        # order + fwd 1 + bwd 1 (both forms when the choice is left to the device) + sh 1.
+        # Counting sort: ranges from the projection's counts 2 + scatter 1 + tile sort 3.
+        # Radix: scan 2 + segments 1 + per group duplicate 1, sort 3/pass, ranges 1 +
+        # segment sort 4 (plan, small, chunk, merge).
+        n_order = _order_launches(T_) * ((order & 1) + ((order >> 1) & 1))
+        grouping = 6 if getattr(self.raster, "binning", 0) else 3 + g * (3 * passes + 2) + 4
+        r = self.raster
+        both = (r.pixels_per_thread_bwd or r.pixels_per_thread) == 2 and T_ >= 65536
+        return 1 + grouping + n_order + 1 + 1 + int(both) + 1
 
     def kernel_stats(self):
         torch.cuda.synchronize()
