@@ -13,6 +13,7 @@
 #pragma once
 
 #include <cuda_bf16.h>
+#include <math_constants.h>
 
 #include "svr_block.cuh"
 #include "svr_common.cuh"
@@ -122,6 +123,41 @@ __device__ __forceinline__ void trilinear_coefficients(const float g[8], float4&
   lo = make_float4(g[0], z0, g[2] - g[0], z1 - z0);
   hi = make_float4(g[4] - g[0], z2 - z0, (g[6] - g[4]) - (g[2] - g[0]), (z3 - z2) - (z1 - z0));
 }
+// The polynomial of densities as they come.  Its coefficients are differences of
+// corners, which infinities turn into NaN (an opaque voxel, and NaN gradients) and
+// corners past half the largest float into infinities; and next to a corner at
+// -1e8 and below the ordinary ones vanish in their rounding.  Such records, seldom
+// met, get coefficients that evaluate as the corners weighted one by one do:
+//   - an infinite (or NaN) corner makes the density that everywhere inside;
+//   - so does a corner that is lower than the others by more than rounding keeps:
+//     the interpolant is far below zero except next to the voxel's far end, in less
+//     than rounding resolves (corners masked with a type's lowest value);
+//   - others are clamped to where differences of differences still fit: only their
+//     sign matters.
+constexpr float kWideDensity = 1e8f, kHugeDensity = 1e37f;
+__device__ __forceinline__ void density_polynomial(float g[8], float4& lo, float4& hi) {
+  float top = 0.f;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) top = fmaxf(top, fabsf(g[c]));
+  if (top >= kWideDensity) {
+    float least = g[0], most = g[0], endless = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      least = fminf(least, g[c]);
+      most = fmaxf(most, g[c]);
+      if (!(fabsf(g[c]) < CUDART_INF_F)) endless += g[c];
+    }
+    const bool empty = least < -kWideDensity * fmaxf(1.f, most);
+    if (endless != 0.f || empty) {
+      lo = make_float4(endless != 0.f ? endless : -CUDART_INF_F, 0.f, 0.f, 0.f);
+      hi = make_float4(0.f, 0.f, 0.f, 0.f);
+      return;
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) g[c] = fminf(fmaxf(g[c], -kHugeDensity), kHugeDensity);
+  }
+  trilinear_coefficients(g, lo, hi);
+}
 __device__ __forceinline__ float trilinear_poly(const float4& lo, const float4& hi, float qx, float qy, float qz) {
   const float a = fmaf(lo.y, qz, lo.x), b = fmaf(lo.w, qz, lo.z);
   const float c = fmaf(hi.y, qz, hi.x), d = fmaf(hi.w, qz, hi.z);
@@ -168,7 +204,7 @@ __device__ __forceinline__ void stage_record(FwdStage<SB>& s, int slot, uint32_t
   float g[8];
   read_densities<MAYBE_GRID>(va, vid, g);
   if (FAST) {
-    trilinear_coefficients(g, s.geo[slot][0], s.geo[slot][1]);
+    density_polynomial(g, s.geo[slot][0], s.geo[slot][1]);
   } else {
     s.geo[slot][0] = make_float4(g[0], g[1], g[2], g[3]);
     s.geo[slot][1] = make_float4(g[4], g[5], g[6], g[7]);
@@ -195,7 +231,7 @@ __device__ __forceinline__ void stage_record(BwdStage<SB>& s, int slot, uint32_t
   float g[8];
   read_densities<MAYBE_GRID>(va, vid, g);
   if (FAST) {
-    trilinear_coefficients(g, s.geo[slot][0], s.geo[slot][1]);
+    density_polynomial(g, s.geo[slot][0], s.geo[slot][1]);
   } else {
     s.geo[slot][0] = make_float4(g[0], g[1], g[2], g[3]);
     s.geo[slot][1] = make_float4(g[4], g[5], g[6], g[7]);
