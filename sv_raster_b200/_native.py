@@ -158,8 +158,14 @@ def check(status, what):
 # What every op does before its launches, kept short: a small view's pass is
 # bounded by this side, and a Stream object, a device guard and a c_void_p per
 # argument took 90 us of a 560 us pass.
+def _need_cuda(dev):
+    if dev.type != "cuda":
+        raise ValueError(f"expected a cuda device, but got: {dev}")
+
+
 def raw_stream(dev):
     """The current CUDA stream of `dev` as a handle the library takes."""
+    _need_cuda(dev)
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if dev.index is None else dev.index)
 
 
@@ -176,6 +182,7 @@ _HERE_ALREADY = _Here()
 
 def on_device(dev):
     """``torch.cuda.device(dev)``, or nothing to do when that device is current."""
+    _need_cuda(dev)
     if dev.index is None or dev.index == torch.cuda.current_device():
         return _HERE_ALREADY
     return torch.cuda.device(dev)
