@@ -348,9 +348,9 @@ def gather_triinterp_geo_params(vox_key, care_idx, grid_pts):
     n_vox = vox_key.size(0)
     out = torch.empty(n_vox, 8, dtype=torch.float32, device=dev)
     with on_device(dev):
-        st = lib().svr_gather_grid_params(1, care_idx.size(0), _ptr(_i64(vox_key, "vox_key")),
-                                          _ptr(_i64(care_idx, "care_idx")), _ptr(_f32(grid_pts, "grid_pts")),
-                                          _ptr(out), _stream(dev))
+        key, care, pts = _i64(vox_key, "vox_key"), _i64(care_idx, "care_idx"), _f32(grid_pts, "grid_pts")
+        st = lib().svr_gather_grid_params(1, care_idx.size(0), _ptr(key), _ptr(care), _ptr(pts), _ptr(out),
+                                          _stream(dev))
     check(st, "gather_triinterp_geo_params")
     return out
 
@@ -360,9 +360,10 @@ def gather_triinterp_geo_params_bw(vox_key, care_idx, num_grid_pts, dL_dgeo_para
     dev = _cuda(dL_dgeo_params, "dL_dgeo_params").device
     out = torch.zeros(int(num_grid_pts), 1, dtype=torch.float32, device=dev)
     with on_device(dev):
-        st = lib().svr_gather_grid_params_bw(1, care_idx.size(0), _ptr(_i64(vox_key, "vox_key")),
-                                             _ptr(_i64(care_idx, "care_idx")),
-                                             _ptr(_f32(dL_dgeo_params, "dL_dgeo_params")), _ptr(out), _stream(dev))
+        key, care = _i64(vox_key, "vox_key"), _i64(care_idx, "care_idx")
+        d = _f32(dL_dgeo_params, "dL_dgeo_params")
+        st = lib().svr_gather_grid_params_bw(1, care_idx.size(0), _ptr(key), _ptr(care), _ptr(d), _ptr(out),
+                                             _stream(dev))
     check(st, "gather_triinterp_geo_params_bw")
     return out
 
@@ -374,9 +375,9 @@ def gather_triinterp_feat_params(vox_key, care_idx, grid_pts):
     dev = _cuda(grid_pts, "grid_pts").device
     out = torch.empty(vox_key.size(0), 8, 3, dtype=torch.float32, device=dev)
     with on_device(dev):
-        st = lib().svr_gather_grid_params(3, care_idx.size(0), _ptr(_i64(vox_key, "vox_key")),
-                                          _ptr(_i64(care_idx, "care_idx")), _ptr(_f32(grid_pts, "grid_pts")),
-                                          _ptr(out), _stream(dev))
+        key, care, pts = _i64(vox_key, "vox_key"), _i64(care_idx, "care_idx"), _f32(grid_pts, "grid_pts")
+        st = lib().svr_gather_grid_params(3, care_idx.size(0), _ptr(key), _ptr(care), _ptr(pts), _ptr(out),
+                                          _stream(dev))
     check(st, "gather_triinterp_feat_params")
     return out
 
@@ -388,9 +389,9 @@ def gather_triinterp_feat_params_bw(vox_key, care_idx, num_grid_pts, dL_dfeat_pa
     dev = _cuda(dL_dfeat_params, "dL_dfeat_params").device
     out = torch.zeros(int(num_grid_pts), 3, dtype=torch.float32, device=dev)
     with on_device(dev):
-        st = lib().svr_gather_grid_params_bw(3, care_idx.size(0), _ptr(_i64(vox_key, "vox_key")),
-                                             _ptr(_i64(care_idx, "care_idx")),
-                                             _ptr(_f32(dL_dfeat_params, "dL_dfeat_params")), _ptr(out),
+        key, care = _i64(vox_key, "vox_key"), _i64(care_idx, "care_idx")
+        d = _f32(dL_dfeat_params, "dL_dfeat_params")
+        st = lib().svr_gather_grid_params_bw(3, care_idx.size(0), _ptr(key), _ptr(care), _ptr(d), _ptr(out),
                                              _stream(dev))
     check(st, "gather_triinterp_feat_params_bw")
     return out

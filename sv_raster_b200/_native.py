@@ -189,5 +189,6 @@ def on_device(dev):
 
 
 def ptr(t):
-    """A tensor's address for a pointer argument (None for no or empty tensors)."""
+    """A tensor's address for a pointer argument (None for no or empty tensors); the
+    caller keeps the tensor, also a copy made for the call, until the call is over."""
     return t.data_ptr() if t is not None and t.numel() > 0 else None

@@ -218,10 +218,10 @@ class BatchedRasterizer:
         if bf16 != (shs.dtype == torch.bfloat16):
             raise ValueError("sh0 and shs must share a dtype")
         M = 1 + shs.shape[1]
+        sh0, shs = sh0.contiguous(), shs.contiguous()  # (copies have to live until the call)
         check(lib().svr_batch_prepare(self.plan, self._p(self.ws), self._p(self.octree_paths), self._p(self.centers),
-                                      self._p(self.lengths), self._p(sh0.contiguous()),
-                                      self._p(shs.contiguous()) if shs.numel() else None, int(bf16), int(sh_degree),
-                                      M, self._stream()), "batch_prepare")
+                                      self._p(self.lengths), self._p(sh0), self._p(shs) if shs.numel() else None,
+                                      int(bf16), int(sh_degree), M, self._stream()), "batch_prepare")
 
     def render(self, geos, out_color=None, out_T=None):
         """Composite every view; returns flat (color [sum 3HW], T [sum HW]).

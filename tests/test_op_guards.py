@@ -71,3 +71,64 @@ def test_streams_and_guards_want_a_cuda_device(a_gpu):
     assert _native.raw_stream(torch.device("cuda")) == 0
     with _native.on_device(torch.device("cuda", 0)):
         pass
+
+
+@pytest.fixture
+def copies(a_gpu, monkeypatch):
+    """Every copy that contiguous() makes, as weak references."""
+    made, plain = [], torch.Tensor.contiguous
+
+    def contiguous(t, *a, **k):
+        out = plain(t, *a, **k)
+        if out is not t:
+            made.append(weakref.ref(out))
+        return out
+
+    monkeypatch.setattr(torch.Tensor, "contiguous", contiguous)
+    monkeypatch.setattr(_C, "_cuda", lambda t, name: t)
+    monkeypatch.setattr(_C, "on_device", lambda dev: _native._HERE_ALREADY)
+    monkeypatch.setattr(_C, "_stream", lambda dev: 0)
+    return made
+
+
+def _raster():
+    r = batched.BatchedRasterizer.__new__(batched.BatchedRasterizer)
+    r.plan, r.dev = None, torch.device("cuda", 0)
+    r.ws = r.octree_paths = r.centers = r.lengths = torch.zeros(4)
+    return r
+
+
+def _strided(*shape, dtype=torch.float32):
+    return torch.zeros(*shape[:-1], 2 * shape[-1], dtype=dtype)[..., ::2]
+
+
+STRIDED_CALLS = {  # the call, the copies it needs
+    "prepare": (lambda: _raster().prepare(torch.zeros(6, 16, 3)[:, 0], torch.zeros(6, 16, 3)[:, 1:], 3), 2),
+    "prepare_bf16": (lambda: _raster().prepare(torch.zeros(6, 16, 3).bfloat16()[:, 0],
+                                               torch.zeros(6, 16, 3).bfloat16()[:, 1:], 3), 2),
+    "gather_geo": (lambda: _C.gather_triinterp_geo_params(_strided(6, 8, dtype=torch.int64),
+                                                          _strided(6, dtype=torch.int64), _strided(9, 1)), 3),
+    "gather_geo_bw": (lambda: _C.gather_triinterp_geo_params_bw(
+        _strided(6, 8, dtype=torch.int64), _strided(6, dtype=torch.int64), 9, _strided(6, 8)), 3),
+    "gather_feat": (lambda: _C.gather_triinterp_feat_params(_strided(6, 8, dtype=torch.int64),
+                                                            _strided(6, dtype=torch.int64), _strided(9, 3)), 3),
+    "gather_feat_bw": (lambda: _C.gather_triinterp_feat_params_bw(
+        _strided(6, 8, dtype=torch.int64), _strided(6, dtype=torch.int64), 9, _strided(6, 8, 3)), 3),
+    "sh_compute": (lambda: _C.sh_compute(0, _strided(6, dtype=torch.int64), _strided(6, 3), _strided(3),
+                                         _strided(6, 3), _strided(6, 1, 3)), 5),
+    "total_variation": (lambda: grid_loss_bw.total_variation(
+        _strided(9, 1), _strided(6, 8, dtype=torch.int64), 1.0, _strided(6), False, False, torch.zeros(9, 1)), 3),
+}
+
+
+@pytest.mark.parametrize("name", sorted(STRIDED_CALLS))
+def test_copies_of_strided_inputs_outlive_the_call(name, copies, monkeypatch):
+    """(A copy that is gone when the next one is made lends it its memory: the
+    kernels would read one input in the place of two.)"""
+    alive = []
+    _library(monkeypatch, _Recorder(lambda: alive.append([ref() is not None for ref in copies])))
+    monkeypatch.setattr(grid_loss_bw, "on_device", lambda dev: _native._HERE_ALREADY)
+    monkeypatch.setattr(grid_loss_bw, "raw_stream", lambda dev: 0)
+    call, n = STRIDED_CALLS[name]
+    call()
+    assert alive == [[True] * n]
