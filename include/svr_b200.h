@@ -259,10 +259,16 @@ int svr_batch_plan_create(int n_views, const svr_camera* cams, int64_t P, int64_
 void svr_batch_plan_destroy(svr_batch_plan* plan);
 /* The plan ranks every (voxel, quadrant) pair once, on the first
  * svr_batch_prepare, from the octree paths it is given (one radix sort of 8P
- * keys); instances are then keyed by that rank position.  The table is
- * rebuilt when prepare sees a different octree_paths pointer or after this
- * call (for paths changed in place). */
+ * keys); instances are then keyed by that rank position.  The tables live in
+ * the workspace, which has to keep its contents between calls.  They are
+ * rebuilt when prepare sees a different workspace or octree_paths pointer or
+ * after this call (for paths changed in place, and for a workspace that was
+ * given back and allocated again or written over); a prepare that is captured
+ * into a graph before they were built builds them in every replay. */
 int svr_batch_plan_invalidate_geometry(svr_batch_plan* plan);
+/* 1 when the next svr_batch_prepare with these pointers finds its tables built,
+ * 0 when it builds them. */
+int svr_batch_plan_positions_ready(const svr_batch_plan* plan, const void* workspace, const int64_t* octree_paths);
 /* Compositing schedule of svr_batch_render / svr_batch_backward: both are
  * persistent launches that take (view, tile) items from a device counter.
  * order_flags bit 0 (forward) / bit 1 (backward), both set by default, rank

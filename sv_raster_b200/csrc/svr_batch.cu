@@ -483,8 +483,9 @@ struct svr_batch_plan {
   int rank_bits;  // compressed Morton rank width (position-table sort)
   int pos_bits;   // bits of a rank position (ceil(log2(8P)))
   int key_bits;   // widest group key (all groups sorted with this many passes)
-  bool pos_ready;                 // rank-position table built for pos_paths
+  bool pos_ready;                 // rank-position tables built for pos_paths in workspace pos_ws
   const int64_t* pos_paths;
+  const void* pos_ws;
   int64_t total_tiles, total_pixels;
   // compositing schedule (svr_batch_plan_set_schedule)
   int order_flags;        // bit 0: forward tiles largest first, bit 1: backward (else tile order)
@@ -615,6 +616,7 @@ int svr_batch_plan_create(int n_views, const svr_camera* cams, int64_t P, int64_
   p->pos_bits = bit_width_u64((uint64_t)(8 * P - 1));
   p->pos_ready = false;
   p->pos_paths = nullptr;
+  p->pos_ws = nullptr;
   p->vt.n = n_views;
   int64_t tiles = 0, pix = 0;
   for (int v = 0; v < n_views; ++v) {
@@ -741,6 +743,10 @@ int svr_batch_plan_invalidate_geometry(svr_batch_plan* p) {
   if (!p) return SVR_ERR_SHAPE;
   p->pos_ready = false;
   return SVR_OK;
+}
+
+int svr_batch_plan_positions_ready(const svr_batch_plan* p, const void* ws, const int64_t* octree_paths) {
+  return p && p->pos_ready && p->pos_ws == ws && p->pos_paths == octree_paths;
 }
 
 int svr_batch_plan_set_schedule(svr_batch_plan* p, int order_flags, int fwd_ctas_per_sm, int bwd_ctas_per_sm) {
@@ -876,7 +882,7 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
 #undef SVR_PROJ
 #undef SVR_PROJ_AS
   // (counting alone, as capacity fitting does, needs no positions)
-  if (p->cap > 0 && (!p->pos_ready || p->pos_paths != octree_paths)) {
+  if (p->cap > 0 && !svr_batch_plan_positions_ready(p, ws, octree_paths)) {
     // Rank positions of all (voxel, quadrant) pairs: one stable radix sort of
     // the 8P compressed ranks in the (still free) instance arrays.
     const size_t n8 = 8 * (size_t)P;
@@ -885,8 +891,13 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
     const int in_b = launch_radix_sort(q.ka, q.va, q.kb, q.vb, nullptr, q.header + 5, (uint32_t)n8, p->rank_bits,
                                        q.sort_tmp, stream);
     rank_pos_scatter_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(n8, in_b ? q.vb : q.va, q.rank_pos, q.val_of_pos);
-    p->pos_ready = true;
+    // The tables are there from now on, unless these launches failed or were only
+    // recorded (a graph that is never replayed builds nothing).
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(stream, &capturing);
+    p->pos_ready = capturing == cudaStreamCaptureStatusNone && cudaPeekAtLastError() == cudaSuccess;
     p->pos_paths = octree_paths;
+    p->pos_ws = ws;
   }
   if (p->binning) {
     // Counting sort by tile: the projection's counts to ranges, every instance's
