@@ -203,11 +203,17 @@ struct PixelRay {
 };
 
 // Y_FIRST: which product of the direction's two-term dot products is rounded
-// before the other is fused onto it.  Written out so that every kernel agrees
-// with its counterpart (the compiler's choice differed between them): true is
-// the reference's order; the batched backward has always had the other one,
-// and its gradients (equally far from their exact values) keep it.
-template <bool Y_FIRST = true>
+// before the other is fused onto it, written out because the compiler's choice
+// differed between kernels.  True is the reference's order, that of every forward
+// and of every backward with exact arithmetic: these have the same rays bit for bit,
+// so the T that a backward recovers record by record arrives at the forward's 1.
+// The batched backward's fast arithmetic has always had the other order and keeps
+// it: its rays differ from its forward's by an ulp here and there, which moves a
+// record's alpha by up to 1e-3 for voxels of 1/4096 and the recovered T with it (4e-3
+// behind a handful of opaque ones).  Either order is equally far from 64 bits over
+// whole gradients; taking the forward's moved single gradients by up to 6e-3 of their
+// norm, which callers who compare runs would see.
+template <bool Y_FIRST>
 __device__ __forceinline__ PixelRay make_pixel_ray(float pixx, float pixy, int W, int H,
                                                    float tanfovx, float tanfovy, float cx, float cy,
                                                    const float* c2w) {

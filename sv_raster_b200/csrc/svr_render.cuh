@@ -347,8 +347,8 @@ __device__ __forceinline__ void place_in_voxel(const PixelRay& r, float t, const
 
 // Fast arithmetic: exp(-optical depth) of a segment from its samples' summed
 // activations.  The backward divides T by 1 - alpha, which for an opaque voxel
-// keeps few digits: it has to arrive at the forward's alpha bit for bit, so both
-// call this.
+// keeps few digits, so both passes call this: from the same ray they arrive at the
+// same alpha bit for bit (make_pixel_ray says how far their rays agree).
 __device__ __forceinline__ float fast_transmittance(float step_sz, float act_sum) {
   return ex2_approx((-kStepScale * kLog2E * step_sz) * act_sum);
 }

@@ -20,11 +20,11 @@ def _every_other(t):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_coefficients_as_slices_of_one_tensor(dtype):
     C = SceneTensors(synthetic.config_scene("c1"))
-    r = _raster(C)
+    r, _ = _raster(C)
     gen = torch.Generator(device="cuda").manual_seed(2)
     # as wide as the scene's own (16 terms), and so narrow that both copies are of a size
     for M, deg in ((16, 3), (2, 0)):
-        both = torch.randn(C.P, M, 3, device="cuda", generator=gen).to(dtype)
+        both = torch.randn(len(C.centers), M, 3, device="cuda", generator=gen).to(dtype)
         r.prepare(both[:, 0].contiguous(), both[:, 1:].contiguous(), deg)
         want = r.arrays()["rgbs"].clone()
         r.arrays()["rgbs"].zero_()
