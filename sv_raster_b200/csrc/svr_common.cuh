@@ -203,17 +203,16 @@ struct PixelRay {
 };
 
 // Y_FIRST: which product of the direction's two-term dot products is rounded
-// before the other is fused onto it, written out because the compiler's choice
-// differed between kernels.  True is the reference's order, that of every forward
-// and of every backward with exact arithmetic: these have the same rays bit for bit,
-// so the T that a backward recovers record by record arrives at the forward's 1.
-// The batched backward's fast arithmetic has always had the other order and keeps
-// it: its rays differ from its forward's by an ulp here and there, which moves a
-// record's alpha by up to 1e-3 for voxels of 1/4096 and the recovered T with it (4e-3
-// behind a handful of opaque ones).  Either order is equally far from 64 bits over
-// whole gradients; taking the forward's moved single gradients by up to 6e-3 of their
-// norm, which callers who compare runs would see.
-template <bool Y_FIRST>
+// before the other is fused onto it.  Written out because the compiler's choice
+// differed between kernels: true is the reference's order, that of every forward
+// and of the plain backward; the batched backward has always had the other one and
+// keeps it.  Its rays differ from its forward's by an ulp here and there, which moves
+// a record's alpha by up to 1e-3 for voxels of 1/4096, and the T that it recovers
+// with it (4e-3 behind a handful of opaque ones, away from the optical axis).  Over
+// whole gradients either order is equally far from 64 bits; the forward's would move
+// single ones by up to 1.4e-3 of their norm (the fast arithmetic's alone, by 1.2e-5
+// from the exact one's).
+template <bool Y_FIRST = true>
 __device__ __forceinline__ PixelRay make_pixel_ray(float pixx, float pixy, int W, int H,
                                                    float tanfovx, float tanfovy, float cx, float cy,
                                                    const float* c2w) {

@@ -46,7 +46,7 @@ __device__ __forceinline__ void render_tile_fwd(const ViewParams& vp, const floa
   const uint32_t px = tile_x * CFG::TS + lx, py = tile_y * CFG::TS + ly;
   const uint32_t pix_id = (uint32_t)W * py + px;
   const bool inside = px < (uint32_t)W && py < (uint32_t)H;
-  const PixelRay ray = make_pixel_ray<true>((float)px, (float)py, W, H, vp.tanfovx, vp.tanfovy, vp.cx, vp.cy, c2w_s);
+  const PixelRay ray = make_pixel_ray((float)px, (float)py, W, H, vp.tanfovx, vp.tanfovy, vp.cx, vp.cy, c2w_s);
   const int warp = tid >> 5;
   const uint32_t wx0 = tile_x * CFG::TS + (warp % CFG::MX) * 8, wy0 = tile_y * CFG::TS + (warp / CFG::MX) * 4;
 

@@ -70,7 +70,7 @@ __device__ __forceinline__ void render_tile_fwd_pair(const ViewParams& vp, const
   for (int k = 0; k < 2; ++k) {
     py[k] = wy0 + (lane >> 3) + 4 * k;
     inside[k] = px < (uint32_t)W && py[k] < (uint32_t)H;
-    ray[k] = make_pixel_ray<true>((float)px, (float)py[k], W, H, vp.tanfovx, vp.tanfovy, vp.cx, vp.cy, c2w_s);
+    ray[k] = make_pixel_ray((float)px, (float)py[k], W, H, vp.tanfovx, vp.tanfovy, vp.cx, vp.cy, c2w_s);
     done[k] = !inside[k];
     T[k] = 1.f;
     Cx[k] = Cy[k] = Cz[k] = 0.f;
@@ -300,7 +300,7 @@ __device__ __forceinline__ void render_tile_bwd_pair(const ViewParams& vp, const
     const uint32_t py = wy0 + (lane >> 3) + 4 * k;
     inside[k] = px < (uint32_t)W && py < (uint32_t)H;
     PairPix& p = pix[k];
-    p.ray = make_pixel_ray<!FAST>((float)px, (float)py, W, H, vp.tanfovx, vp.tanfovy, vp.cx, vp.cy, c2w_s);
+    p.ray = make_pixel_ray<false>((float)px, (float)py, W, H, vp.tanfovx, vp.tanfovy, vp.cx, vp.cy, c2w_s);
     const uint32_t pix_id = (uint32_t)W * py + px;
     p.T = inside[k] ? in.T[pix_id] : 0.f;
     last_contrib[k] = inside[k] ? in.n_contrib[pix_id] : 0u;
