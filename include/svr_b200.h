@@ -339,6 +339,10 @@ int svr_batch_plan_set_pixels_per_thread(svr_batch_plan* plan, int pixels);
  * pixel's own records with one pixel per thread; the backward walks a list with
  * all lanes on one record with two, so the best choices can differ. */
 int svr_batch_plan_set_backward_pixels_per_thread(svr_batch_plan* plan, int pixels);
+/* 1 (default): svr_batch_backward also looks at the sizes, takes one pixel per
+ * thread where two were set but are slower (above) and stages 64 records where
+ * 32 were set for at most 4,500 tiles of 8x8.  0: as set, whatever the sizes. */
+int svr_batch_plan_set_backward_adaptive(svr_batch_plan* plan, int adaptive);
 int64_t svr_batch_plan_pixels(const svr_batch_plan* plan);
 int64_t svr_batch_plan_tiles(const svr_batch_plan* plan);
 int svr_batch_plan_groups(const svr_batch_plan* plan);

@@ -60,6 +60,7 @@ class BatchedRasterizer:
         self.exact = bool(exact)
         self.pixels_per_thread = 1
         self.pixels_per_thread_bwd = None  # None: as pixels_per_thread
+        self.backward_adaptive = True
         self.culling = -1  # -1: tight bbox with the fast arithmetic, the rounded one with the exact
         self.staging_bwd = None  # None: the forward's staging depth
         self._make_plan(0 if capacity is None else int(capacity))
@@ -92,6 +93,8 @@ class BatchedRasterizer:
               "batch_plan_set_pixels_per_thread")
         check(L.svr_batch_plan_set_backward_pixels_per_thread(plan, self.pixels_per_thread_bwd or 0),
               "batch_plan_set_backward_pixels_per_thread")
+        check(L.svr_batch_plan_set_backward_adaptive(plan, int(self.backward_adaptive)),
+              "batch_plan_set_backward_adaptive")
         if self.staging_bwd is not None:
             check(L.svr_batch_plan_set_backward_staging(plan, self.staging_bwd), "batch_plan_set_backward_staging")
 
@@ -140,6 +143,14 @@ class BatchedRasterizer:
         check(lib().svr_batch_plan_set_backward_pixels_per_thread(self.plan, int(pixels or 0)),
               "batch_plan_set_backward_pixels_per_thread")
         self.pixels_per_thread_bwd = int(pixels) if pixels else None
+
+    def set_backward_adaptive(self, adaptive=True):
+        """Whether the backward also looks at the sizes before it takes the
+        pixels per thread and the staging depth that were set (see
+        svr_batch_plan_set_backward_adaptive); False: exactly as set."""
+        check(lib().svr_batch_plan_set_backward_adaptive(self.plan, int(bool(adaptive))),
+              "batch_plan_set_backward_adaptive")
+        self.backward_adaptive = bool(adaptive)
 
     def set_tile_size(self, tile_size, staging=None):
         """Compositing tile size (8, 16 or 32 pixels) and records staged per

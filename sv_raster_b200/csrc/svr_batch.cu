@@ -498,6 +498,7 @@ struct svr_batch_plan {
   int exact;                   // compositing arithmetic (svr_batch_plan_set_arithmetic): 1 exact, 0 fast
   int pair;                    // two pixels per compositing thread (svr_batch_plan_set_pixels_per_thread)
   int pair_bwd;                // the backward's, when set apart (-1: as pair)
+  int adaptive;                // the backward's form and staging also by size (svr_batch_plan_set_backward_adaptive)
   int culling;                 // pixel bbox (svr_batch_plan_set_culling): -1 follows exact, 0 rounded, 1 tight
   int binning;                 // 1: counting sort by tile, 0: radix over the tile bits (svr_batch_plan_set_binning)
   // workspace layout (byte offsets)
@@ -726,6 +727,7 @@ int svr_batch_plan_create(int n_views, const svr_camera* cams, int64_t P, int64_
   p->exact = 0;
   p->pair = 0;
   p->pair_bwd = -1;
+  p->adaptive = 1;
   p->culling = -1;
   p->binning = 1;
   ensure_segsort_attributes();
@@ -782,6 +784,12 @@ int svr_batch_plan_set_pixels_per_thread(svr_batch_plan* p, int pixels) {
 int svr_batch_plan_set_backward_pixels_per_thread(svr_batch_plan* p, int pixels) {
   if (!p || pixels < 0 || pixels > 2) return SVR_ERR_SHAPE;
   p->pair_bwd = pixels == 0 ? -1 : (pixels == 2);
+  return SVR_OK;
+}
+
+int svr_batch_plan_set_backward_adaptive(svr_batch_plan* p, int adaptive) {
+  if (!p || (adaptive != 0 && adaptive != 1)) return SVR_ERR_SHAPE;
+  p->adaptive = adaptive;
   return SVR_OK;
 }
 
@@ -974,7 +982,7 @@ static int batch_backward(svr_batch_plan* p, void* ws, VoxelArrays va, const flo
   else cudaMemsetAsync(q.header + 3, 0, sizeof(uint32_t), stream);
   launch_render_bwd_batch(p->vt, (int)p->total_tiles, q.ranges, q.tile_last, p->cap > 0 ? q.vb : nullptr, va,
                           (int)p->P, (size_t)p->P * 3, (size_t)p->P * 4, in, out, p->n_samp, p->tile_size,
-                          p->stage_bwd, !p->exact, p->pair_bwd < 0 ? p->pair : p->pair_bwd,
+                          p->stage_bwd, !p->exact, p->pair_bwd < 0 ? p->pair : p->pair_bwd, p->adaptive != 0,
                           CoverageCount{coverage_words(q), q.header}, ordered ? q.order_bwd : nullptr, q.header + 3,
                           p->bwd_ctas_per_sm, stream);
   return check_last();

@@ -113,7 +113,7 @@ void launch_render_bwd(const ViewParams& vp, const uint2* ranges, const uint32_t
 void launch_render_bwd_batch(const ViewTable& views, int n_items, const uint2* ranges,
                              const uint32_t* tile_last, const uint32_t* vals, const VoxelArrays& va, int P,
                              size_t rgb_view_stride, size_t drgb_view_stride, const BwdTileIn& in,
-                             const BwdTileOut& out, int ns, int tile, int stage, bool fast, int pair,
+                             const BwdTileOut& out, int ns, int tile, int stage, bool fast, int pair, bool adaptive,
                              const CoverageCount& coverage, const uint32_t* order, uint32_t* counter, int ctas_per_sm,
                              cudaStream_t stream);
 // svr_binning_deep.cu: binning of 21-level octrees (63-bit ranks).  The sort

@@ -277,7 +277,7 @@ static void launch_bwd_batch_cfg(const BwdBatchArgs& args, int ns, bool fast, in
 void launch_render_bwd_batch(const ViewTable& views, int n_items, const uint2* ranges,
                              const uint32_t* tile_last, const uint32_t* vals, const VoxelArrays& va, int P,
                              size_t rgb_view_stride, size_t drgb_view_stride, const BwdTileIn& in,
-                             const BwdTileOut& out, int ns, int tile, int stage, bool fast, int pair,
+                             const BwdTileOut& out, int ns, int tile, int stage, bool fast, int pair, bool adaptive,
                              const CoverageCount& coverage, const uint32_t* order, uint32_t* counter, int ctas_per_sm,
                              cudaStream_t stream) {
   if (n_items <= 0) return;
@@ -294,19 +294,21 @@ void launch_render_bwd_batch(const ViewTable& views, int n_items, const uint2* r
   // tiles at 18 pixels 0.24 / 0.31 ms; 10,000 tiles at 5 pixels 2.5 / 4.5 ms.  So
   // the two-pixel form takes many tiles (their lists overlap each other's tails)
   // of broad records; how broad they are is known on the device alone, and the
-  // form that is not wanted returns at once.
-  if (pair && batch_pair_supported(tile, stage) && n_items >= kManyTiles) {
-    args.run_when = 1;
+  // form that is not wanted returns at once.  (Not adaptive: the form and the depth
+  // that were set, whatever the sizes.)
+  if (pair && batch_pair_supported(tile, stage) && (n_items >= kManyTiles || !adaptive)) {
+    args.run_when = adaptive ? 1 : -1;
     if (tile == 8 && stage == 32) launch_bwd_pair_cfg<PairCfg<8, 32>>(args, ns, fast, ctas_per_sm, stream);
     else if (tile == 8) launch_bwd_pair_cfg<PairCfg<8, 64>>(args, ns, fast, ctas_per_sm, stream);
     else if (stage == 128) launch_bwd_pair_cfg<PairCfg<16, 128>>(args, ns, fast, ctas_per_sm, stream);
     else launch_bwd_pair_cfg<PairCfg<16, 256>>(args, ns, fast, ctas_per_sm, stream);
+    if (!adaptive) return;
     args.run_when = 0;
   }
   // With few tiles a pass lasts as long as its longest list: 64 records a round
   // halve the rounds' latencies (1,280 tiles of up to 20,000 records 5.5 -> 4.6 ms;
   // from 5,000 tiles on, where more CTAs of 32 records fit, 1.02 times slower).
-  if (tile == 8 && stage == 32 && n_items <= kFewTiles) stage = 64;
+  if (adaptive && tile == 8 && stage == 32 && n_items <= kFewTiles) stage = 64;
   if (tile == 8 && stage == 32) launch_bwd_batch_cfg<TileCfg<8, 32>>(args, ns, fast, ctas_per_sm, stream);
   else if (tile == 8 && stage == 128) launch_bwd_batch_cfg<TileCfg<8, 128>>(args, ns, fast, ctas_per_sm, stream);
   else if (tile == 8) launch_bwd_batch_cfg<TileCfg<8, 64>>(args, ns, fast, ctas_per_sm, stream);
