@@ -199,12 +199,15 @@ project_sh_kernel(const __grid_constant__ ViewTable views, int P, const float* _
 // them.  Places past the capacity are left out (the range scan flagged it).
 // Pairs of few tiles keep their atomics in flight together; a warp takes the
 // others tile by tile, one per lane.  Bound by the returning atomics: 60M
-// instances in 1.16 ms, where a lane per instance, decoded from a scan of all
-// pairs, with keys and values to store took 1.46 and the scan 0.35.
+// instances in 1.15 ms, where a lane per instance, decoded from a scan of all
+// pairs, with keys and values to store took 1.46 and the scan 0.35.  A pair whose
+// tiles and quadrants are not the instances that the projection stored for it is
+// flagged, as the other duplications do.
 __global__ void __launch_bounds__(256)
 scatter_positions_kernel(const __grid_constant__ ViewTable views, int P, const uint32_t* __restrict__ rank_pos,
                          const uint2* __restrict__ bboxes, const uint32_t* __restrict__ quads,
-                         uint32_t* __restrict__ cursor, uint32_t* __restrict__ keys, uint32_t cap) {
+                         const uint32_t* __restrict__ ndup, uint32_t* __restrict__ cursor,
+                         uint32_t* __restrict__ keys, uint32_t cap, uint32_t* __restrict__ err) {
   const ViewParams& vp = views.v[blockIdx.y];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -212,6 +215,7 @@ scatter_positions_kernel(const __grid_constant__ ViewTable views, int P, const u
   const uint32_t qb = i < P ? quads[o] : 0u;
   if (__ballot_sync(0xffffffffu, qb != 0u) == 0u) return;
   const TileRect rect(qb ? bboxes[o] : make_uint2(0u, 0u), vp, qb != 0u);
+  if (qb && rect.n * (uint32_t)__popc(qb) != ndup[o]) atomicOr(err, SVR_DEVERR_DUP_MISMATCH);
   uint32_t* c = cursor + vp.tile_base;
   if (rect.n <= kOwnTiles) {
     for (uint32_t qs = qb; qs; qs &= qs - 1) {
@@ -914,8 +918,8 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
     launch_tile_ranges_from_counts(q.counts, (int)p->total_tiles, (uint32_t)p->cap, q.ranges, q.header, q.header + 1,
                                    q.scan_tmp, q.sort_tmp, q.header + 6, stream);
     if (p->cap > 0) {
-      scatter_positions_kernel<<<grid, 256, 0, stream>>>(p->vt, P, q.rank_pos, q.bbox, q.quad, q.counts, keys,
-                                                         (uint32_t)p->cap);
+      scatter_positions_kernel<<<grid, 256, 0, stream>>>(p->vt, P, q.rank_pos, q.bbox, q.quad, q.ndup, q.counts,
+                                                         keys, (uint32_t)p->cap, q.header + 1);
       launch_tile_sort(q.ranges, (int)p->total_tiles, keys, q.val_of_pos, q.vb, p->cap, q.sort_tmp, q.header + 6,
                        stream);
     }
