@@ -18,6 +18,7 @@
 #include "svr_block.cuh"
 #include "svr_common.cuh"
 #include "svr_kernels.h"
+#include "svr_runs.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -35,6 +36,10 @@ constexpr int kRunWarps = 4;               // 8: 826 us where 4 take 459 and the
 constexpr int kRun = kWarpKeys * kRunWarps;  // keys of one sorted run of a long segment
 constexpr int kTileWarps = 4;
 constexpr int kMergeT = 512;
+// Segments of more runs are merged by windows: 25 runs 2.2 -> 1.6 ms (20M instances), 6
+// to 10 runs by rank 1.05, by windows 1.09 (all of prepare, 2.2M instances).
+constexpr uint32_t kManyRuns = 16;
+using MergeWindow = WindowSmem<kMergeT, 2816>;
 
 }  // namespace
 
@@ -193,9 +198,42 @@ __device__ __forceinline__ int merge_split(const uint32_t* a, int na, const uint
   return lo;
 }
 
-// One CTA per listed run: its warps sort kWarpKeys each, then runs are merged
-// pairwise in shared memory, every thread taking 16 consecutive outputs.  The run
-// of a one-run segment is final; others go back in place for the merge below.
+// Merges sorted runs of len keys in s, n keys in all (padded with 0xffffffff to T * PER),
+// pairwise until one is left, every thread taking PER consecutive outputs.  Starts with
+// a barrier.
+template <int T, int PER>
+__device__ __forceinline__ void merge_in_shared(uint32_t* s, int len, int n) {
+  const int d0 = threadIdx.x * PER;             // first output
+  for (; len < n; len <<= 1) {
+    __syncthreads();
+    uint32_t out[PER];
+    const int pair = d0 & ~(2 * len - 1);       // the two runs [pair, pair + len), [pair + len, pair + 2 len)
+    const uint32_t* a = s + pair;
+    const uint32_t* b = a + len;
+    int i = merge_split(a, len, b, len, d0 - pair), j = d0 - pair - i;
+    // the heads stay in registers; an exhausted run's is the padding key, which
+    // no key is above
+    uint32_t x = i < len ? a[i] : 0xffffffffu, y = j < len ? b[j] : 0xffffffffu;
+#pragma unroll
+    for (int o = 0; o < PER; ++o) {
+      const bool from_a = x <= y;
+      out[o] = min(x, y);
+      i += from_a;
+      j += !from_a;
+      const bool more = (from_a ? i : j) < len;
+      const uint32_t next = more ? (from_a ? a[i] : b[j]) : 0xffffffffu;
+      x = from_a ? next : x;
+      y = from_a ? y : next;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int o = 0; o < PER; o += 4)
+      reinterpret_cast<uint4*>(s + d0)[o / 4] = make_uint4(out[o], out[o + 1], out[o + 2], out[o + 3]);
+  }
+}
+
+// One CTA per listed run: its warps sort kWarpKeys each, then those are merged.  The
+// run of a one-run segment is final; others go back in place for the merge below.
 __global__ void __launch_bounds__(32 * kRunWarps)
 sort_runs_kernel(const uint4* __restrict__ runs, const uint32_t* __restrict__ n_runs, uint32_t runs_cap,
                  uint32_t* __restrict__ keys, const uint32_t* __restrict__ val_of_pos, uint32_t* __restrict__ vals) {
@@ -208,33 +246,7 @@ sort_runs_kernel(const uint4* __restrict__ runs, const uint32_t* __restrict__ n_
     const int n = (int)run.y;
     warp_sort_to_shared<kWarpKeys / 32>(keys + run.x + warp * kWarpKeys, max(0, n - warp * kWarpKeys),
                                         s + warp * kWarpKeys, lane);
-    for (int len = kWarpKeys; len < n; len <<= 1) {
-      __syncthreads();
-      uint32_t out[PER];
-      const int d0 = tid * PER;                 // first output
-      const int pair = d0 & ~(2 * len - 1);     // the two runs [pair, pair + len), [pair + len, pair + 2 len)
-      const uint32_t* a = s + pair;
-      const uint32_t* b = a + len;
-      int i = merge_split(a, len, b, len, d0 - pair), j = d0 - pair - i;
-      // the heads stay in registers; an exhausted run's is the padding key, which
-      // no key is above
-      uint32_t x = i < len ? a[i] : 0xffffffffu, y = j < len ? b[j] : 0xffffffffu;
-#pragma unroll
-      for (int o = 0; o < PER; ++o) {
-        const bool from_a = x <= y;
-        out[o] = min(x, y);
-        i += from_a;
-        j += !from_a;
-        const bool more = (from_a ? i : j) < len;
-        const uint32_t next = more ? (from_a ? a[i] : b[j]) : 0xffffffffu;
-        x = from_a ? next : x;
-        y = from_a ? y : next;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int o = 0; o < PER; o += 4)
-        reinterpret_cast<uint4*>(s + d0)[o / 4] = make_uint4(out[o], out[o + 1], out[o + 2], out[o + 3]);
-    }
+    merge_in_shared<32 * kRunWarps, PER>(s, kWarpKeys, n);
     __syncthreads();
     if (run.w == run.y) {
       for (int i = tid; i < n; i += 32 * kRunWarps) vals[run.x + i] = val_of_pos[s[i]];
@@ -246,12 +258,15 @@ sort_runs_kernel(const uint4* __restrict__ runs, const uint32_t* __restrict__ n_
 }
 
 // One CTA per run of a longer segment: a key's place is its index in its run
-// plus, for every other run, the number of that run's keys below it.
-__global__ void __launch_bounds__(kMergeT)
+// plus, for every other run, the number of that run's keys below it.  That takes
+// time with the square of the runs, so segments of many are merged by windows of as
+// many keys instead (svr_runs.cuh).
+__global__ void __launch_bounds__(kMergeT, 4)
 merge_runs_kernel(const uint4* __restrict__ runs, const uint32_t* __restrict__ n_runs, uint32_t runs_cap,
                   const uint32_t* __restrict__ keys, const uint32_t* __restrict__ val_of_pos,
                   uint32_t* __restrict__ vals) {
-  __shared__ uint32_t s_other[kRun];
+  __shared__ __align__(16) uint32_t s_other[kRun];
+  __shared__ MergeWindow s_window;
   constexpr int PER = kRun / kMergeT;
   const uint32_t count = min(*n_runs, runs_cap);
   const int tid = threadIdx.x;
@@ -260,6 +275,26 @@ merge_runs_kernel(const uint4* __restrict__ runs, const uint32_t* __restrict__ n
     if (run.w == run.y) continue;  // already final (uniform over the CTA)
     const int n = (int)run.y;
     const uint32_t r = (run.x - run.z) / kRun, k = (run.w + kRun - 1) / kRun;
+    if (k > kManyRuns) {  // (window r has as many keys as run r)
+      gather_window<kMergeT>(SortedRuns<uint32_t, uint32_t>{keys + run.z, run.w, kRun}, r * kRun, r * kRun + n,
+                             s_window, [&](uint32_t i, uint32_t, uint32_t key) { s_other[i] = key; });
+      for (int i = n + tid; i < kRun; i += kMergeT) s_other[i] = 0xffffffffu;
+      __syncthreads();
+      uint32_t* mine = s_other + (tid >> 5) * 32 * PER;
+      const int lane = tid & 31;
+      uint32_t x[PER];
+#pragma unroll
+      for (int o = 0; o < PER; ++o) x[o] = mine[o * 32 + lane];
+      warp_sort(x, lane);
+      __syncwarp();
+#pragma unroll
+      for (int o = 0; o < PER; ++o) mine[lane * PER + o] = x[o];
+      merge_in_shared<kMergeT, PER>(s_other, 32 * PER, n);
+      __syncthreads();
+      for (int i = tid; i < n; i += kMergeT) vals[run.x + i] = val_of_pos[s_other[i]];
+      __syncthreads();
+      continue;
+    }
     uint32_t own[PER], below[PER];
 #pragma unroll
     for (int o = 0; o < PER; ++o) {
