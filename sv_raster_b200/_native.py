@@ -160,8 +160,11 @@ def check(status, what):
 # What every op does before its launches, kept short: a small view's pass is
 # bounded by this side, and a Stream object, a device guard and a c_void_p per
 # argument took 90 us of a 560 us pass.
+_CUDA = frozenset([torch.device("cuda")] + [torch.device("cuda", i) for i in range(128)])
+
+
 def _need_cuda(dev):
-    if dev.type != "cuda":
+    if dev not in _CUDA:  # (dev.type is a new string each time: 180 ns against 40)
         raise ValueError(f"expected a cuda device, but got: {dev}")
 
 
