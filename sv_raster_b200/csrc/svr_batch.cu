@@ -80,6 +80,15 @@ struct TileRect {
   }
 };
 
+// Copies of the tile counts (and of the scatter's cursors): with many voxels over few
+// tiles their atomics meet in a handful of cache lines.  n copies (a power of two),
+// stride words apart; 128 consecutive voxels share one.  20M voxels, 64 tiles: the
+// projection with its counts 4.98 -> 0.62 ms, the scatter 5.01 -> 0.29.
+struct TileCopies {
+  uint32_t n, stride;
+  __device__ __forceinline__ uint32_t offset(uint32_t voxel) const { return (voxel / 128u & (n - 1u)) * stride; }
+};
+
 // View-dependent colour of a visible voxel (sh_compute.cu:54-106); m holds the
 // view's w2c and c2w.
 template <int DEG, typename TS>
@@ -98,7 +107,7 @@ __device__ __forceinline__ void view_colour(const float* m, float cx, float cy, 
 // With `counts`, every visible pair also adds its instances to its tiles' counts
 // (a warp takes the pairs of many tiles together, one tile per lane): 1.78 -> 2.22
 // ms (before SH_LAST) for 8M voxels and eight views, where counting in a pass of its own, which
-// re-read 20 bytes per pair, took 0.88.
+// re-read 20 bytes per pair, took 0.88.  Blocks take the counts' copies in turn (TileCopies).
 //
 // SH_LAST (two views and more): the colours follow all projections, with the
 // coefficients in registers, so they are read once for all views, all in flight
@@ -113,7 +122,8 @@ project_sh_kernel(const __grid_constant__ ViewTable views, int P, const float* _
                   const float* __restrict__ lengths, const TS* __restrict__ sh0, const TS* __restrict__ shs, int M,
                   const int64_t* __restrict__ octpaths, int level_low_bits, int tight, uint32_t* __restrict__ ndup,
                   uint2* __restrict__ bboxes, uint32_t* __restrict__ quads, float* __restrict__ rgbs,
-                  uint32_t* __restrict__ err, unsigned long long* __restrict__ pixels, uint32_t* __restrict__ counts) {
+                  uint32_t* __restrict__ err, unsigned long long* __restrict__ pixels, uint32_t* __restrict__ counts,
+                  const TileCopies copies) {
   __shared__ float s_m[kMaxViews][24];           // w2c (12) and c2w (12) of every view
   __shared__ unsigned long long s_pixels;
   if (threadIdx.x == 0) s_pixels = 0ull;
@@ -147,7 +157,7 @@ project_sh_kernel(const __grid_constant__ ViewTable views, int P, const float* _
     if (counts) {
       const TileRect rect(pr.bbox, views.v[v], visible);
       const uint32_t per_tile = (uint32_t)__popc(pr.quads);
-      uint32_t* c = counts + views.v[v].tile_base;
+      uint32_t* c = counts + copies.offset(blockIdx.x * blockDim.x) + views.v[v].tile_base;
       if (rect.n <= kOwnTiles) {
         uint32_t t = rect.first, left = rect.w;
         for (uint32_t k = 0; k < rect.n; ++k) {
@@ -203,11 +213,14 @@ project_sh_kernel(const __grid_constant__ ViewTable views, int P, const float* _
 // pairs, with keys and values to store took 1.46 and the scan 0.35.  A pair whose
 // tiles and quadrants are not the instances that the projection stored for it is
 // flagged, as the other duplications do.
+// With copies, cursor[copy][tile] counts from the copy's first place in the tile, whose
+// own is start[tile]; without (start is null) it holds the place itself.
 __global__ void __launch_bounds__(256)
 scatter_positions_kernel(const __grid_constant__ ViewTable views, int P, const uint32_t* __restrict__ rank_pos,
                          const uint2* __restrict__ bboxes, const uint32_t* __restrict__ quads,
                          const uint32_t* __restrict__ ndup, uint32_t* __restrict__ cursor,
-                         uint32_t* __restrict__ keys, uint32_t cap, uint32_t* __restrict__ err) {
+                         const TileCopies copies, const uint32_t* __restrict__ start, uint32_t* __restrict__ keys,
+                         uint32_t cap, uint32_t* __restrict__ err) {
   const ViewParams& vp = views.v[blockIdx.y];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -216,7 +229,8 @@ scatter_positions_kernel(const __grid_constant__ ViewTable views, int P, const u
   if (__ballot_sync(0xffffffffu, qb != 0u) == 0u) return;
   const TileRect rect(qb ? bboxes[o] : make_uint2(0u, 0u), vp, qb != 0u);
   if (qb && rect.n * (uint32_t)__popc(qb) != ndup[o]) atomicOr(err, SVR_DEVERR_DUP_MISMATCH);
-  uint32_t* c = cursor + vp.tile_base;
+  uint32_t* c = cursor + copies.offset((uint32_t)(i - lane)) + vp.tile_base;
+  const auto place = [&](uint32_t t) { return atomicAdd(c + t, 1u) + (start ? start[vp.tile_base + t] : 0u); };
   if (rect.n <= kOwnTiles) {
     for (uint32_t qs = qb; qs; qs &= qs - 1) {
       const uint32_t pos = rank_pos[8 * (size_t)i + (__ffs(qs) - 1)];
@@ -224,7 +238,7 @@ scatter_positions_kernel(const __grid_constant__ ViewTable views, int P, const u
       uint32_t t = rect.first, left = rect.w;
 #pragma unroll
       for (uint32_t k = 0; k < kOwnTiles; ++k) {
-        if (k < rect.n) at[k] = atomicAdd(c + t, 1u);
+        if (k < rect.n) at[k] = place(t);
         ++t;
         if (--left == 0) {
           left = rect.w;
@@ -243,7 +257,7 @@ scatter_positions_kernel(const __grid_constant__ ViewTable views, int P, const u
     for (uint32_t qs = __shfl_sync(0xffffffffu, qb, src); qs; qs &= qs - 1) {
       const uint32_t pos = rank_pos[8 * vox + (__ffs(qs) - 1)];
       for (uint32_t k = lane; k < r.n; k += 32) {
-        const uint32_t at = atomicAdd(c + r.tile(k), 1u);
+        const uint32_t at = place(r.tile(k));
         if (at < cap) keys[at] = pos;
       }
     }
@@ -502,13 +516,14 @@ struct svr_batch_plan {
   int exact;                   // compositing arithmetic (svr_batch_plan_set_arithmetic): 1 exact, 0 fast
   int pair;                    // two pixels per compositing thread (svr_batch_plan_set_pixels_per_thread)
   int pair_bwd;                // the backward's, when set apart (-1: as pair)
+  TileCopies copies;           // of the counting sort's tile counts
   int adaptive;                // the backward's form and staging also by size (svr_batch_plan_set_backward_adaptive)
   int culling;                 // pixel bbox (svr_batch_plan_set_culling): -1 follows exact, 0 rounded, 1 tight
   int binning;                 // 1: counting sort by tile, 0: radix over the tile bits (svr_batch_plan_set_binning)
   // workspace layout (byte offsets)
   size_t o_header, o_ndup, o_scan, o_bbox, o_quad, o_scan_tmp, o_rgbs, o_drgbs;
   size_t o_ka, o_kb, o_va, o_vb, o_sort_tmp, o_ranges, o_tile_last, o_ncontrib;
-  size_t o_okey, o_oval, o_order_fwd, o_order_bwd, o_order_tmp, o_pos, o_valpos;
+  size_t o_okey, o_oval, o_order_fwd, o_order_bwd, o_order_tmp, o_pos, o_valpos, o_copies;
   size_t bytes;
 };
 
@@ -537,6 +552,7 @@ struct BatchPtrs {
   uint32_t* rank_pos;   // [8P] position of (voxel, quadrant) in rank order
   uint32_t* val_of_pos; // [8P] instance value of a position
   uint32_t* counts;     // [T] instances per tile, then the scatter's cursors (after the header)
+  uint32_t* copies;     // [copies.n][copies.stride] their copies, when there are several
 };
 
 // Header words: [0] instance count, [1] error word, [2] forward work counter,
@@ -574,11 +590,25 @@ BatchPtrs ptrs(const svr_batch_plan* p, void* ws) {
   q.rank_pos = reinterpret_cast<uint32_t*>(b + p->o_pos);
   q.val_of_pos = reinterpret_cast<uint32_t*>(b + p->o_valpos);
   q.counts = q.header + kHeaderWords;
+  q.copies = reinterpret_cast<uint32_t*>(b + p->o_copies);
   return q;
 }
 
 unsigned long long* coverage_words(const BatchPtrs& q) {
   return reinterpret_cast<unsigned long long*>(q.header + kCoverageWord);
+}
+
+// Several copies where a view has at least 256 voxels per tile: as many as spread its
+// counters over 32,768 words, where they help no more.  All of prepare, without and with:
+// 2M voxels on 64 tiles 1.21 / 0.33 ms, on 1,024 0.64 / 0.23, on 4,096 (490 a tile) 0.30 /
+// 0.22; with under 256 a tile the counters lie far enough apart by themselves.
+TileCopies tile_copies(const ViewTable& vt, int64_t total_tiles, int64_t P) {
+  int64_t fewest = total_tiles;
+  for (int v = 0; v < vt.n; ++v) fewest = std::min(fewest, (int64_t)vt.v[v].grid_x * vt.v[v].grid_y);
+  uint32_t n = 1;
+  if (P >= 256 * fewest)
+    while (n < 64 && 2 * n * fewest <= 32768) n *= 2;
+  return TileCopies{n, (uint32_t)((total_tiles + 31) / 32 * 32)};
 }
 
 // Largest-first work order of all tiles into `order`, and the work counter back
@@ -722,6 +752,8 @@ int svr_batch_plan_create(int n_views, const svr_camera* cams, int64_t P, int64_
   p->o_order_tmp = take(sort_temp_bytes((size_t)tiles));
   p->o_pos = take((size_t)(8 * P) * 4);
   p->o_valpos = take((size_t)(8 * P) * 4);
+  p->copies = tile_copies(p->vt, tiles, P);
+  p->o_copies = take(p->copies.n > 1 ? (size_t)p->copies.n * p->copies.stride * 4 : 0);
   p->bytes = align_up(off) + kAlign;
   p->order_flags = 3;
   p->fwd_ctas_per_sm = 0;
@@ -868,14 +900,17 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
   const int P = (int)p->P;
   const size_t VP = (size_t)p->V * p->P;
   cudaMemsetAsync(q.header, 0, (kHeaderWords + (size_t)p->total_tiles) * sizeof(uint32_t), stream);
-  uint32_t* counts = p->binning ? q.counts : nullptr;
+  const bool copied = p->binning && p->copies.n > 1;
+  uint32_t* counts = p->binning ? (copied ? q.copies : q.counts) : nullptr;
+  if (copied) cudaMemsetAsync(q.copies, 0, (size_t)p->copies.n * p->copies.stride * sizeof(uint32_t), stream);
   const dim3 pgrid((P + 127) / 128);
   const int level_low = (p->rank_bits == kRankBits) ? 0 : kRankBits - (p->rank_bits - 3);  // 3*(16-L)
   const int tight = p->culling < 0 ? !p->exact : p->culling;
 #define SVR_PROJ_AS(D, TS, LAST)                                                                              \
   project_sh_kernel<D, TS, LAST><<<pgrid, 128, 0, stream>>>(                                                  \
       p->vt, P, vox_centers, vox_lengths, (const TS*)sh0, (const TS*)shs, M, octree_paths, level_low, tight,  \
-      q.ndup, q.bbox, q.quad, q.rgbs, q.header + 1, coverage_words(q), counts)
+      q.ndup, q.bbox, q.quad, q.rgbs, q.header + 1, coverage_words(q), counts,           \
+      p->copies)
 #define SVR_PROJ(D)                                                                                           \
   if (sh_bf16) {                                                                                              \
     if (p->V > 1) SVR_PROJ_AS(D, __nv_bfloat16, true);                                                        \
@@ -915,11 +950,13 @@ int svr_batch_prepare(svr_batch_plan* p, void* ws, const int64_t* octree_paths, 
     // Counting sort by tile: the projection's counts to ranges, every instance's
     // rank position scattered into its tile's range, each range sorted.
     uint32_t* keys = reinterpret_cast<uint32_t*>(q.ka);
+    if (copied) launch_tile_copies(q.copies, (int)p->copies.n, p->copies.stride, (int)p->total_tiles, q.counts, stream);
     launch_tile_ranges_from_counts(q.counts, (int)p->total_tiles, (uint32_t)p->cap, q.ranges, q.header, q.header + 1,
                                    q.scan_tmp, q.sort_tmp, q.header + 6, stream);
     if (p->cap > 0) {
-      scatter_positions_kernel<<<grid, 256, 0, stream>>>(p->vt, P, q.rank_pos, q.bbox, q.quad, q.ndup, q.counts,
-                                                         keys, (uint32_t)p->cap, q.header + 1);
+      scatter_positions_kernel<<<grid, 256, 0, stream>>>(p->vt, P, q.rank_pos, q.bbox, q.quad, q.ndup, counts,
+                                                         p->copies, copied ? q.counts : nullptr, keys,
+                                                         (uint32_t)p->cap, q.header + 1);
       launch_tile_sort(q.ranges, (int)p->total_tiles, keys, q.val_of_pos, q.vb, p->cap, q.sort_tmp, q.header + 6,
                        stream);
     }

@@ -72,6 +72,10 @@ void launch_tile_ranges(const uint64_t* keys, const uint32_t* d_start, const uin
 // counts[n_tiles] become the scatter cursors; n_runs is one device word, zero at
 // the call; scan_temp and run_list hold tile_scan_temp_bytes / tile_sort_temp_bytes.
 size_t tile_scan_temp_bytes(int n_tiles);
+// Up to 64 copies of the tile counts, stride words apart: their sums to counts, and every
+// copy's first place within its tile in its stead.
+void launch_tile_copies(uint32_t* copies, int n_copies, uint32_t stride, int n_tiles, uint32_t* counts,
+                        cudaStream_t stream);
 size_t tile_sort_temp_bytes(size_t cap, int n_tiles);
 void launch_tile_ranges_from_counts(uint32_t* counts, int n_tiles, uint32_t cap, uint2* ranges, uint32_t* d_total,
                                     uint32_t* err, void* scan_temp, void* run_list, uint32_t* n_runs,

@@ -69,6 +69,33 @@ tile_counts_reduce_kernel(const uint32_t* __restrict__ counts, int n, unsigned l
   if (threadIdx.x == 0) sums[blockIdx.x] = tot;
 }
 
+// One warp per tile.
+__global__ void __launch_bounds__(256)
+tile_copies_kernel(uint32_t* __restrict__ copies, int n_copies, uint32_t stride, int n_tiles,
+                   uint32_t* __restrict__ counts) {
+  const int lane = threadIdx.x & 31, t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (t >= n_tiles) return;
+  uint32_t before = 0;
+  for (int c0 = 0; c0 < n_copies; c0 += 32) {
+    const int c = c0 + lane;
+    const uint32_t x = c < n_copies ? copies[c * stride + t] : 0u;
+    uint32_t incl = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (c < n_copies) copies[c * stride + t] = before + incl - x;
+    before += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) counts[t] = before;
+}
+
+void launch_tile_copies(uint32_t* copies, int n_copies, uint32_t stride, int n_tiles, uint32_t* counts,
+                        cudaStream_t stream) {
+  tile_copies_kernel<<<(n_tiles + 7) / 8, 256, 0, stream>>>(copies, n_copies, stride, n_tiles, counts);
+}
+
 // Ranges [start, end) of every tile, clamped to the capacity, empty ones (0, 0);
 // counts[t] becomes the tile's scatter cursor.  The last CTA stores the instance
 // count and flags one past the capacity.  Tiles longer than a warp sorts are

@@ -126,3 +126,36 @@ def test_keys_with_values_are_the_stable_sort(levels, n, size, twice):
     vals = q << 29 | vox
     assert R == vals.numel()
     assert torch.equal(got, vals[_sorted_by(t, _ranks(path.reshape(-1), vals, levels))])
+
+
+@pytest.mark.parametrize("capacity", [None, 50_000])
+@pytest.mark.parametrize("sizes,n", [([(24, 16)], 1_535), ([(24, 16)], 1_536), ([(24, 16), (8, 8), (40, 24)], 4_096),
+                                     ([(24, 16), (40, 24)], 300_000), ([(256, 256)], 600_000),
+                                     ([(720, 360)], 1_100_000)])
+def test_copies_of_the_counts(sizes, n, capacity):
+    """On both sides of 256 voxels per tile of a view, from where the counting sort's
+    counts and cursors are kept in copies: the lists of the radix binning, and within a
+    capacity that is too small lists that keep to it, with the error word set."""
+    path, _, centers, lengths = _cells(n, n + 2)
+    cams = [_Cam(synthetic.make_camera(*s, 30.0, (0.3 - 0.2 * k, -0.2, -2.0))) for k, s in enumerate(sizes)]
+    sh0, shs = torch.zeros(n, 3).cuda(), torch.zeros(n, 0, 3).cuda()
+    got = []
+    for binning in (1, 0):
+        r = BatchedRasterizer(cams, path, centers, lengths, max_level=LEVEL, tile_size=8, capacity=capacity)
+        r.set_culling(0)
+        r.set_binning(binning)
+        if capacity is None:
+            r.fit_capacity(sh0, shs, 0)
+        r.prepare(sh0, shs, 0)
+        total, err = r.header()
+        a = r.arrays()
+        if capacity is not None and total > capacity:
+            assert err == 4  # capacity
+            if binning:
+                rg = a["ranges"].long()
+                assert (rg[:, 1] <= capacity).all() and (rg[:, 1] - rg[:, 0]).sum() == capacity
+            continue
+        assert err == 0
+        got.append((a["ranges"].clone(), a["sorted_vals"][:total].clone()))
+    if got:
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
