@@ -203,14 +203,15 @@ __device__ __forceinline__ void stage_record(FwdStage<SB>& s, int slot, uint32_t
   s.corner[slot] = make_float4(cx - rad, cy - rad, cz - rad, 1.f / len);
   float g[8];
   read_densities<MAYBE_GRID>(va, vid, g);
+  const float* rgb = va.rgbs + 3 * (size_t)vid;
+  const float red = rgb[0], green = rgb[1], blue = rgb[2];  // (under way before the densities are looked at)
   if (FAST) {
     density_polynomial(g, s.geo[slot][0], s.geo[slot][1]);
   } else {
     s.geo[slot][0] = make_float4(g[0], g[1], g[2], g[3]);
     s.geo[slot][1] = make_float4(g[4], g[5], g[6], g[7]);
   }
-  const float* rgb = va.rgbs + 3 * (size_t)vid;
-  s.rgb[slot] = make_float4(rgb[0], rgb[1], rgb[2], __int_as_float((int)vid));
+  s.rgb[slot] = make_float4(red, green, blue, __int_as_float((int)vid));
 }
 
 template <bool FAST, bool MAYBE_GRID, int SB>
@@ -230,14 +231,15 @@ __device__ __forceinline__ void stage_record(BwdStage<SB>& s, int slot, uint32_t
   s.corner[slot] = make_float4(cx - rad, cy - rad, cz - rad, __int_as_float((int)vid));
   float g[8];
   read_densities<MAYBE_GRID>(va, vid, g);
+  const float* rgb = va.rgbs + 3 * (size_t)vid;
+  const float red = rgb[0], green = rgb[1], blue = rgb[2];  // (under way before the densities are looked at)
   if (FAST) {
     density_polynomial(g, s.geo[slot][0], s.geo[slot][1]);
   } else {
     s.geo[slot][0] = make_float4(g[0], g[1], g[2], g[3]);
     s.geo[slot][1] = make_float4(g[4], g[5], g[6], g[7]);
   }
-  const float* rgb = va.rgbs + 3 * (size_t)vid;
-  s.rgb[slot] = make_float4(rgb[0], rgb[1], rgb[2], 0.f);
+  s.rgb[slot] = make_float4(red, green, blue, 0.f);
 }
 
 // A plain CTA composites an 8x8 block but walks the list of the 16x16 tile
