@@ -92,10 +92,13 @@ def test_one_tile_of_all_voxels(n):
 
 @pytest.mark.parametrize("levels", [16, 21])
 @pytest.mark.parametrize("n,size,twice", [(65_536, (16, 16), False), (70_000, (16, 16), True),
-                                          (400_000, (16, 16), False), (300_000, (32, 16), True)])
+                                          (200_000, (16, 16), False), (262_000, (16, 16), True),
+                                          (263_000, (16, 16), True), (400_000, (16, 16), False),
+                                          (300_000, (32, 16), True), (600_000, (32, 16), True)])
 def test_keys_with_values_are_the_stable_sort(levels, n, size, twice):
     """Single views of one and two 16x16 tiles.  `twice`: half of the voxels have another's
-    path, so equal keys must keep the order in which they were generated."""
+    path, so equal keys must keep the order in which they were generated.  21 levels: on
+    both sides of the lists that are sorted by rank first (262,144 instances a tile)."""
     path16, path21, centers, lengths = _cells(n, n + 1)
     path = path16 if levels == 16 else path21
     if twice:
