@@ -112,3 +112,33 @@ def test_deep_keys_are_the_stable_sort(n_chains, size):
     assert np.array_equal(lo.cpu().numpy().view(np.uint64), tile << np.uint64(63) | rank)
     assert np.array_equal(hi.cpu().numpy().view(np.uint64), tile >> np.uint64(1))
     assert np.array_equal(vals.cpu().numpy().view(np.uint32), (inst[:, 2] << 29 | inst[:, 1]).astype(np.uint32))
+
+
+@pytest.mark.parametrize("n,views", [(262_144, 64), (262_145, 64), (600_000, 40)])
+def test_scan_of_many_pairs(n, views):
+    """The radix binning's scan over (view, voxel) pairs on both sides of the 16.7M from
+    which its CTAs' sums are scanned first, and past them: its total is the counts', and
+    the lists are the counting sort's."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    k = torch.randperm(1 << 21, device="cuda", generator=gen)[:n]
+    ijk = torch.stack([k >> 14, (k >> 7) & 127, k & 127], 1)
+    path = torch.zeros_like(k)
+    for b in range(7):
+        o = (ijk >> b) & 1
+        path |= (o[:, 0] * 4 + o[:, 1] * 2 + o[:, 2]) << (3 * b)
+    centers = ((ijk.float() + 0.5) / 128 - 0.5).contiguous()
+    cams = [_Cam(synthetic.make_camera(40, 24, 40.0, (0.05 * v, -0.2, -2.0))) for v in range(views)]
+    sh0, shs = torch.zeros(n, 3).cuda(), torch.zeros(n, 0, 3).cuda()
+    got = []
+    for binning in (0, 1):
+        r = BatchedRasterizer(cams, path << 27, centers, torch.full((n, 1), 1 / 128, device="cuda"), max_level=7,
+                              tile_size=8)
+        r.set_binning(binning)
+        total = r.fit_capacity(sh0, shs, 0)
+        r.prepare(sh0, shs, 0)
+        assert r.header() == (total, 0)
+        a = r.arrays()
+        assert total == int(a["ndup"].long().sum())
+        got.append((a["ranges"].clone(), a["sorted_vals"][:total].clone()))
+        del r
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
