@@ -10,9 +10,9 @@
 // stable sort of the wide key gives.  Sorting all instances by rank first, in seven
 // radix passes, and then stably by tile gives it too, in a time that does not depend on
 // how long the tiles' lists are: 300k voxels, 801x601, all of binning 158 us where 77 are
-// taken; 20M voxels on 256 tiles (82,000 instances each) 4.58 and 4.55 ms; on 64 tiles
-// (321,000) 4.45 and 4.60; on one 4.3 and 36.  So lists that are long on average are
-// sorted by rank first.
+// taken; 2M voxels on 144 tiles (15,000 instances each) 409 and 380 us, on 64 (33,000) 403
+// and 449; 20M on 256 tiles (82,000) 4.23 and 4.54 ms, on 16 (1.3M) 4.1 and 6.5, on one
+// 4.0 and 36.  So lists that are long on average are sorted by rank first.
 // The wide keys (as lo = tile << 63 | rank, hi = tile >> 1, the reference's
 // SortKey128 halves), the sorted values and the tile ranges are left where the
 // 16-level path leaves its own, so compositing and its backward read them
@@ -28,7 +28,7 @@ __host__ __device__ constexpr uint64_t octant_repeat_deep(uint64_t q) {
   return v;
 }
 
-constexpr uint32_t kLongLists = 1u << 16;  // instances per tile on average
+constexpr uint32_t kLongLists = 1u << 15;  // instances per tile on average
 
 // One (tile, index) pair per instance in generation order (forward.cu:518-571
 // of new_cuda, with the instance's own index as the carried value), plus the

@@ -91,20 +91,21 @@ def test_one_tile_of_all_voxels(n):
 
 
 @pytest.mark.parametrize("levels", [16, 21])
-@pytest.mark.parametrize("n,size,twice", [(65_536, (16, 16), False), (70_000, (16, 16), True),
-                                          (200_000, (16, 16), False), (262_000, (16, 16), True),
-                                          (263_000, (16, 16), True), (400_000, (16, 16), False),
-                                          (300_000, (32, 16), True), (600_000, (32, 16), True)])
-def test_keys_with_values_are_the_stable_sort(levels, n, size, twice):
-    """Single views of one and two 16x16 tiles.  `twice`: half of the voxels have another's
-    path, so equal keys must keep the order in which they were generated.  21 levels: on
-    both sides of the lists that are sorted by rank first (262,144 instances a tile)."""
+@pytest.mark.parametrize("n,size,dist,twice", [
+    (25_000, (16, 16), 3.0, True), (32_700, (16, 16), 3.0, False), (65_536, (16, 16), 3.0, False),
+    (70_000, (16, 16), 3.0, True), (400_000, (16, 16), 3.0, False), (300_000, (32, 16), 3.0, True),
+    (150_000, (512, 16), 60.0, False), (200_000, (512, 16), 60.0, True)])
+def test_keys_with_values_are_the_stable_sort(levels, n, size, dist, twice):
+    """Single views of one and two 16x16 tiles, and of 32 of which two hold everything.
+    `twice`: half of the voxels have another's path, so equal keys must keep the order in
+    which they were generated.  21 levels: by tile first and (from 32,768 instances per
+    tile on average) by rank first."""
     path16, path21, centers, lengths = _cells(n, n + 1)
     path = path16 if levels == 16 else path21
     if twice:
         path = path[torch.arange(n, device="cuda") // 2 * 2].contiguous()
     C = mC if levels == 16 else dC
-    cam = _Cam(synthetic.make_camera(*size, 40.0, (0.3, -0.2, -3.0)))
+    cam = _Cam(synthetic.make_camera(*size, 40.0, (0.3, -0.2, -dist)))
     a = (cam.width, cam.height, cam.tanfovx, cam.tanfovy, cam.cx, cam.cy, cam.w2c, cam.c2w)
     p = path.reshape(-1, 1)
     ndup, geom = C.rasterize_preprocess(*a, cam.near, p, centers, lengths)
