@@ -146,10 +146,6 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
 // lands on the early-stop threshold.
 constexpr float kLog2E = 1.4426950408889634f;
 template <bool FAST>
-__device__ __forceinline__ float exp_f(float x) {
-  return FAST ? ex2_approx(x * kLog2E) : expf(x);
-}
-template <bool FAST>
 __device__ __forceinline__ float div_f(float a, float b) {
   return FAST ? a * rcp_approx(b) : a / b;
 }

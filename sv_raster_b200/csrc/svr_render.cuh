@@ -49,9 +49,11 @@ constexpr int kFwdMinBlocks = 4;
 constexpr int kBwdMinBlocks = 3;
 template <class CFG>
 constexpr int fwd_min_blocks() { return CFG::NT >= 1024 ? 1 : kFwdMinBlocks * 256 / CFG::NT; }
-// The one-pixel backward: its CTAs of 64 threads run 13 (32 staged records) or
-// 11 (64) to an SM, at up to 78 or 90 registers (16 at 64 registers: the plain
-// backward 1.69 -> 2.08 ms on a 2M-voxel view).
+// The one-pixel backward: its CTAs of 64 threads run 14 (32 staged records) or 12 (64)
+// to an SM, which the bounds of 13 and 11 come to: the compiler rounds to 72 and 80
+// registers.  Nothing spills with one sample and fast arithmetic; the plain forms spill
+// 20 to 136 bytes but for the simplest (16 CTAs at 64 registers: the plain backward 1.69
+// -> 2.08 ms on a 2M-voxel view).
 template <class CFG>
 constexpr int bwd_min_blocks() {
   return CFG::NT >= 1024 ? 1 : (CFG::NT == 64 ? (CFG::SB <= 32 ? 13 : 11) : kBwdMinBlocks * 256 / CFG::NT);

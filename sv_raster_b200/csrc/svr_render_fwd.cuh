@@ -31,7 +31,7 @@ struct FwdTileOut {
 // `last_slot` receives range.x + the tile's largest contributor count, with
 // atomicMax when SHARED_LIST (several CTAs share one list, read through s_list,
 // and one slot, which then starts at 0).
-// FAST selects the arithmetic of the per-(pixel, voxel) loop (exp_f, svr_common.cuh).
+// FAST selects the arithmetic of the per-(pixel, voxel) loop (act_exp_f, svr_common.cuh).
 template <class CFG, int NS, bool DEPTH, bool DIST, bool NORMAL, bool MAXW, bool SHARED_LIST = false, bool FAST = false>
 __device__ __forceinline__ void render_tile_fwd(const ViewParams& vp, const float* __restrict__ c2w_s, int tile_x,
                                                 int tile_y, uint2 range, const uint32_t* __restrict__ vals,

@@ -5,10 +5,9 @@
 // Together this yields exactly the order of one stable sort by the full
 // [tile | rank] key (forward.cu:678-686): the tile passes keep generation
 // order inside a tile, and every step below orders by rank with generation
-// order breaking ties.  The batched path may group by tile with a counting
-// sort instead, which leaves a tile's instances in no particular order; its
-// keys (rank positions) are unique inside a tile, so the sorted result is the
-// same.
+// order breaking ties.  Used by the plain path, by the batched path's radix
+// grouping (its counting sort has a tile sort of its own, svr_tilesort.cu) and by
+// the grouping by tile of 21-level octrees (svr_binning_deep.cu).
 //
 // Tile sizes are heavy-tailed (in a dense 1080p scene the median tile holds a
 // few hundred instances while a few percent of the tiles hold tens of

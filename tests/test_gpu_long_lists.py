@@ -135,7 +135,7 @@ def test_keys_with_values_are_the_stable_sort(levels, n, size, dist, twice):
 @pytest.mark.parametrize("capacity", [None, 50_000])
 @pytest.mark.parametrize("sizes,n", [([(24, 16)], 1_535), ([(24, 16)], 1_536), ([(24, 16), (8, 8), (40, 24)], 4_096),
                                      ([(24, 16), (40, 24)], 300_000), ([(256, 256)], 600_000),
-                                     ([(720, 360)], 1_100_000)])
+                                     ([(720, 360)], 1_100_000), ([(8, 8), (360, 200)], 150_000)])
 def test_copies_of_the_counts(sizes, n, capacity):
     """On both sides of 256 voxels per tile of a view, from where the counting sort's
     counts and cursors are kept in copies: the lists of the radix binning, and within a
