@@ -598,17 +598,18 @@ unsigned long long* coverage_words(const BatchPtrs& q) {
   return reinterpret_cast<unsigned long long*>(q.header + kCoverageWord);
 }
 
-// Several copies where there are at least 256 voxels per tile of a view (on average:
-// that bounds their memory): as many as spread a view's counters over 32,768 words,
-// where they help no more.  All of prepare, without and with:
-// 2M voxels on 64 tiles 1.21 / 0.33 ms, on 1,024 0.64 / 0.23, on 4,096 (490 a tile) 0.30 /
-// 0.22; with under 256 a tile the counters lie far enough apart by themselves.
-TileCopies tile_copies(int n_views, int64_t total_tiles, int64_t P) {
-  const int64_t per_view = (total_tiles + n_views - 1) / n_views;
-  uint32_t n = 1;
-  if (P >= 256 * per_view)
-    while (n < 64 && 2 * n * per_view <= 32768) n *= 2;
-  return TileCopies{n, (uint32_t)((total_tiles + 31) / 32 * 32)};
+// Several copies where the smallest view has at least 256 voxels per tile: as many as
+// spread its counters over 32,768 words, where they help no more, and within a million
+// words for all views.  All of prepare, without and with: 2M voxels on 64 tiles 1.21 /
+// 0.33 ms, on 1,024 0.64 / 0.23, on 4,096 (490 a tile) 0.30 / 0.22; a step of 2M voxels
+// and 16 views of 640x480 to 1600x1200 (four copies) 11.70 / 11.34.
+TileCopies tile_copies(const ViewTable& vt, int64_t total_tiles, int64_t P) {
+  int64_t fewest = total_tiles;
+  for (int v = 0; v < vt.n; ++v) fewest = std::min(fewest, (int64_t)vt.v[v].grid_x * vt.v[v].grid_y);
+  int64_t n = 1;
+  if (P >= 256 * fewest)
+    while (n < 64 && 2 * n * fewest <= 32768 && 2 * n * total_tiles <= 1 << 20) n *= 2;
+  return TileCopies{(uint32_t)n, (uint32_t)((total_tiles + 31) / 32 * 32)};
 }
 
 // Largest-first work order of all tiles into `order`, and the work counter back
@@ -752,7 +753,7 @@ int svr_batch_plan_create(int n_views, const svr_camera* cams, int64_t P, int64_
   p->o_order_tmp = take(sort_temp_bytes((size_t)tiles));
   p->o_pos = take((size_t)(8 * P) * 4);
   p->o_valpos = take((size_t)(8 * P) * 4);
-  p->copies = tile_copies(n_views, tiles, P);
+  p->copies = tile_copies(p->vt, tiles, P);
   p->o_copies = take(p->copies.n > 1 ? (size_t)p->copies.n * p->copies.stride * 4 : 0);
   p->bytes = align_up(off) + kAlign;
   p->order_flags = 3;
