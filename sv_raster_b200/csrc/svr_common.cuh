@@ -206,8 +206,8 @@ struct PixelRay {
 // a record's alpha by up to 1e-3 for voxels of 1/4096, and the T that it recovers
 // with it (4e-3 behind a handful of opaque ones, away from the optical axis).  Over
 // whole gradients either order is equally far from 64 bits; the forward's would move
-// single ones by up to 1.4e-3 of their norm, and taken for the exact arithmetic alone
-// the two arithmetics 1.2e-5 apart.
+// single ones by up to 1.4e-3 of their root mean square, and taken for the exact
+// arithmetic alone it would move the two arithmetics 1.2e-5 apart.
 template <bool Y_FIRST = true>
 __device__ __forceinline__ PixelRay make_pixel_ray(float pixx, float pixy, int W, int H,
                                                    float tanfovx, float tanfovy, float cx, float cy,

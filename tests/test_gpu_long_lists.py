@@ -12,7 +12,6 @@ from sv_raster_b200.levels21 import _C as dC
 
 pytestmark = pytest.mark.gpu
 
-LEVEL = 7
 
 
 class _Cam:
@@ -21,19 +20,24 @@ class _Cam:
         self.w2c, self.c2w = (torch.from_numpy(m).cuda() for m in (c.w2c, c.c2w))
 
 
+def _level(n):
+    """The coarsest grid, 128^3 and up, with n cells."""
+    return next(lv for lv in range(7, 16) if n <= 1 << (3 * lv))
+
+
 def _cells(n, seed):
-    """n cells of a 128^3 grid in random order: (octree path of 16 levels, of 21, centres,
+    """n cells of that grid in random order: (octree path of 16 levels, of 21, centres,
     lengths)."""
-    gen = torch.Generator(device="cuda").manual_seed(seed)
-    k = torch.randperm(1 << (3 * LEVEL), device="cuda", generator=gen)[:n]
-    ijk = torch.stack([k >> (2 * LEVEL), (k >> LEVEL) & 127, k & 127], 1)
+    gen, lv = torch.Generator(device="cuda").manual_seed(seed), _level(n)
+    k = torch.randperm(1 << (3 * lv), device="cuda", generator=gen)[:n]
+    ijk = torch.stack([k >> (2 * lv), (k >> lv) & ((1 << lv) - 1), k & ((1 << lv) - 1)], 1)
     path = torch.zeros_like(k)
-    for b in range(LEVEL):
+    for b in range(lv):
         oct_ = ((ijk >> b) & 1)
         path |= (oct_[:, 0] * 4 + oct_[:, 1] * 2 + oct_[:, 2]) << (3 * b)
-    centers = ((ijk.float() + 0.5) / (1 << LEVEL) - 0.5).contiguous()
-    return (path << (3 * (16 - LEVEL)), path << (3 * (21 - LEVEL)), centers,
-            torch.full((n, 1), 1.0 / (1 << LEVEL), device="cuda"))
+    centers = ((ijk.float() + 0.5) / (1 << lv) - 0.5).contiguous()
+    return (path << (3 * (16 - lv)), path << (3 * (21 - lv)), centers,
+            torch.full((n, 1), 1.0 / (1 << lv), device="cuda"))
 
 
 def _sorted_by(tile, rank):
@@ -54,8 +58,9 @@ def _ranks(path, vals, levels):
 
 
 # around the number of runs (16 of 2,048 positions; 16 of 4,096 keys, or of 2,048) from
-# which windows merge, whole and partial last runs, and hundreds of runs
-SIZES = [18_432, 32_768, 32_769, 40_000, 65_536, 65_537, 400_000, 1_500_000]
+# which windows merge, whole and partial last runs, hundreds of runs, and more (2,816 of
+# positions, 2,432 of 2,048 keys) than a window keeps track of
+SIZES = [18_432, 32_768, 32_769, 40_000, 65_536, 65_537, 400_000, 1_500_000, 6_500_000]
 
 
 @pytest.mark.parametrize("n", SIZES)
@@ -68,7 +73,7 @@ def test_one_tile_of_all_voxels(n):
     sh0, shs = torch.zeros(n, 3).cuda(), torch.zeros(n, 0, 3).cuda()
     lists = []
     for binning, buckets in ((1, (512, 4096)), (0, (512, 4096)), (0, (512, 2048))):
-        r = BatchedRasterizer([cam], path, centers, lengths, max_level=LEVEL, tile_size=8)
+        r = BatchedRasterizer([cam], path, centers, lengths, max_level=_level(n), tile_size=8)
         r.set_culling(0)
         r.set_binning(binning)
         r.set_sort_buckets(*buckets)
@@ -94,7 +99,8 @@ def test_one_tile_of_all_voxels(n):
 @pytest.mark.parametrize("n,size,dist,twice", [
     (25_000, (16, 16), 3.0, True), (32_700, (16, 16), 3.0, False), (65_536, (16, 16), 3.0, False),
     (70_000, (16, 16), 3.0, True), (400_000, (16, 16), 3.0, False), (300_000, (32, 16), 3.0, True),
-    (150_000, (512, 16), 60.0, False), (200_000, (512, 16), 60.0, True)])
+    (150_000, (512, 16), 60.0, False), (200_000, (512, 16), 60.0, True),
+    (21_500_000, (16, 16), 3.0, True)])  # more runs (5,152 of 4,096 keys) than a window keeps track of
 def test_keys_with_values_are_the_stable_sort(levels, n, size, dist, twice):
     """Single views of one and two 16x16 tiles, and of 32 of which two hold everything.
     `twice`: half of the voxels have another's path, so equal keys must keep the order in
@@ -145,7 +151,7 @@ def test_copies_of_the_counts(sizes, n, capacity):
     sh0, shs = torch.zeros(n, 3).cuda(), torch.zeros(n, 0, 3).cuda()
     got = []
     for binning in (1, 0):
-        r = BatchedRasterizer(cams, path, centers, lengths, max_level=LEVEL, tile_size=8, capacity=capacity)
+        r = BatchedRasterizer(cams, path, centers, lengths, max_level=_level(n), tile_size=8, capacity=capacity)
         r.set_culling(0)
         r.set_binning(binning)
         if capacity is None:
