@@ -403,14 +403,14 @@ class BatchedWorkload:
         # project 1 + grouping by tile and sort + per ordered compositing stage its tile
         # order + fwd 1 + bwd 1 (both forms when the choice is left to the device) + sh 1.
         # Counting sort: ranges from the projection's counts 2 + scatter 1 + tile sort 3,
-        # and the sum of the counts' copies with at least 256 voxels per tile of the smallest view.
+        # and the sum of the counts' copies with many voxels per tile.
         # Radix: scan 2 + segments 1 + per group duplicate 1, sort 3/pass, ranges 1 +
         # segment sort 4 (plan, small, chunk, merge).
         n_order = _order_launches(T_) * ((order & 1) + ((order >> 1) & 1))
         r = self.raster
         ts = r.tile_size
         fewest = min(math.ceil(h / ts) * math.ceil(w / ts) for h, w in r.sizes)
-        copies = int(r.P >= 256 * fewest and 2 * fewest <= 32768 and 2 * T_ <= 1 << 20)
+        copies = int(r.P >= max(65536, 256 * fewest) and 2 * fewest <= 32768 and 2 * T_ <= 1 << 20)
         grouping = 6 + copies if getattr(r, "binning", 0) else 3 + g * (3 * passes + 2) + 4
         both = (r.pixels_per_thread_bwd or r.pixels_per_thread) == 2 and T_ >= 65536
         return 1 + grouping + n_order + 1 + 1 + int(both) + 1

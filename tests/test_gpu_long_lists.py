@@ -139,11 +139,12 @@ def test_keys_with_values_are_the_stable_sort(levels, n, size, dist, twice):
 
 
 @pytest.mark.parametrize("capacity", [None, 50_000])
-@pytest.mark.parametrize("sizes,n", [([(24, 16)], 1_535), ([(24, 16)], 1_536), ([(24, 16), (8, 8), (40, 24)], 4_096),
+@pytest.mark.parametrize("sizes,n", [([(24, 16)], 65_535), ([(24, 16)], 65_536), ([(320, 160)], 204_799),
+                                     ([(320, 160)], 204_800), ([(24, 16), (8, 8), (40, 24)], 70_000),
                                      ([(24, 16), (40, 24)], 300_000), ([(256, 256)], 600_000),
                                      ([(720, 360)], 1_100_000), ([(8, 8), (360, 200)], 150_000)])
 def test_copies_of_the_counts(sizes, n, capacity):
-    """On both sides of 256 voxels per tile of a view, from where the counting sort's
+    """On both sides of 65,536 voxels and of 256 per tile, from where the counting sort's
     counts and cursors are kept in copies: the lists of the radix binning, and within a
     capacity that is too small lists that keep to it, with the error word set."""
     path, _, centers, lengths = _cells(n, n + 2)
